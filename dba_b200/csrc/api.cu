@@ -183,6 +183,8 @@ MBP<R> mb_params(dba_ctx* c, bool dba_mode)
     P.Mx = k.mob_x; P.My = k.mob_y; P.Mz = k.mob_z; P.k0 = k.k_0;
     P.thr = k.metric_eps;
     P.conserved = (k.conserved && dba_mode) ? 1 : 0;
+    auto exact_rcp = [](int r) { return r > 0 && (r & (r - 1)) == 0 ? 1.0 / r : 0.0; };
+    P.irx = exact_rcp(k.rx); P.iry = exact_rcp(k.ry); P.irz = exact_rcp(k.rz);
     return P;
 }
 
@@ -855,9 +857,11 @@ int dba_init_f32(dba_ctx* c, const float* ic)
         for (size_t i = 0; i < m; ++i) tmp[i] = ic[i];
         return dba_init(c, tmp.data());
     }
-    // FP32 dendrite and Model B: the state fields go to the device as they are
+    // FP32 dendrite and Model B: the state fields go to the device as they are.  The clears are
+    // ordered on the context's stream like the copies: a clear on the default stream does not
+    // wait for the stream and may still run when the first copy writes the field it clears
     DBA_TRY(cudaStreamSynchronize(c->st));
-    for (auto& a : c->allocs) DBA_TRY(cudaMemset(a.p, 0, a.bytes));
+    for (auto& a : c->allocs) DBA_TRY(cudaMemsetAsync(a.p, 0, a.bytes, c->st));
     for (int q = 0; q < c->nstate; ++q)
         DBA_TRY(cudaMemcpyAsync(c->state[q][0], ic + q * c->n, c->n * sizeof(float), cudaMemcpyHostToDevice, c->st));
     // step 1 reads wake[1 % 3]: every block starts active (as dba_init)
