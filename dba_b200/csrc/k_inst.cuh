@@ -13,20 +13,6 @@ static int grid_of(const void* kern, size_t smem, int sms)
     return occ * sms;
 }
 
-template <typename R, int D, int B>
-static bool mb_prepare(size_t& smem)
-{
-    smem = MBShape<R, D, B>::smem;
-    if (smem > 200 * 1024) return false;
-    static bool done[2] = {false, false};
-    if (!done[0]) {
-        done[0] = true;
-        cudaFuncSetAttribute(modelb_step<R, D, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(modelb_step<R, D, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
-    return true;
-}
-
 #define DBA_DEN_SHAPES(X) X(2, 4) X(2, 8) X(2, 16) X(2, 32) X(3, 4) X(3, 8)
 #define DBA_MB_SHAPES(X) X(2, 4) X(2, 8) X(2, 16) X(2, 32) X(3, 4) X(3, 8)
 #define DBA_KH_SHAPES(X) X(4) X(8) X(16)
@@ -44,13 +30,26 @@ bool shape_supported(int model, int D, int B)
     return false;
 }
 
+// the two-kernel Model B step: shared-memory limits on the current device, and the grid of
+// the correction pass
+template <typename R, int D, int B>
+static int mb_prepare(int sms)
+{
+    using S = MBShape<R, D, B>;
+    cudaFuncSetAttribute(modelb_mu<R, D, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    cudaFuncSetAttribute(modelb_mu<R, D, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    cudaFuncSetAttribute(modelb_update<R, D, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_cons);
+    cudaFuncSetAttribute(modelb_update<R, D, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    return grid_of<R>((const void*)cons_correct<R>, 0, sms);
+}
+
 template <typename R>
 int step_grid(int model, int D, int B, int sms)
 {
 #define XD(d, b) if (D == d && B == b) return grid_of<R>((const void*)dendrite_step<R, d, b, true>, 0, sms);
-#define XM(d, b) if (D == d && B == b) { size_t sm; mb_prepare<R, d, b>(sm); \
+#define XM(d, b) if (D == d && B == b) { \
     if constexpr (sizeof(R) == 4 && d == 2) return grid_of<R>((const void*)modelb_fast_step<b, true>, MBFastShape<b>::smem, sms); \
-    return grid_of<R>((const void*)modelb_step<R, d, b, true>, sm, sms); }
+    else return mb_prepare<R, d, b>(sms); }
 #define XK(b) if (B == b) return grid_of<R>((const void*)kh_extrap<R, b, true>, 0, sms);
     if (model == MODEL_DENDRITE) { DBA_DEN_SHAPES(XD) }
     if (model == MODEL_MODELB) { DBA_MB_SHAPES(XM) }
@@ -82,6 +81,23 @@ bool modelb_uses_fast(int D, int B)
     return sizeof(R) == 4 && D == 2 && (B == 4 || B == 8 || B == 16 || B == 32);
 }
 
+// one CTA per tile; potentials, then the update
+template <typename R, int D, int B>
+static cudaError_t mb_split(bool dba_mode, cudaStream_t st, const GridP& g, const FlagP& f, const MBP<R>& P)
+{
+    using S = MBShape<R, D, B>;
+    const int nt = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY) * (D == 3 ? (g.nz + S::TZ - 1) / S::TZ : 1);
+    const size_t sc = P.conserved ? S::smem_cons : S::smem_mu;
+    if (dba_mode) {
+        modelb_mu<R, D, B, true><<<nt, S::NT, S::smem_mu, st>>>(g, f, P);
+        modelb_update<R, D, B, true><<<nt, S::NT, sc, st>>>(g, f, P);
+    } else {
+        modelb_mu<R, D, B, false><<<nt, S::NT, S::smem_mu, st>>>(g, f, P);
+        modelb_update<R, D, B, false><<<nt, S::NT, sc, st>>>(g, f, P);
+    }
+    return cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t launch_modelb(int D, int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                           const MBP<R>& P, const LazyP* lz, int tiles)
@@ -105,17 +121,13 @@ cudaError_t launch_modelb(int D, int B, bool dba_mode, int grid, cudaStream_t st
         }
     }
 #define XM(d, b)                                                                            \
-    if (D == d && B == b) {                                                                 \
-        size_t sm;                                                                          \
-        if (!mb_prepare<R, d, b>(sm)) return cudaErrorInvalidValue;                         \
-        if (dba_mode) modelb_step<R, d, b, true><<<grid, kThreads, sm, st>>>(g, f, P);      \
-        else modelb_step<R, d, b, false><<<grid, kThreads, sm, st>>>(g, f, P);              \
-        return cudaGetLastError();                                                          \
-    }
+    if constexpr (!(sizeof(R) == 4 && d == 2))                                              \
+        if (D == d && B == b) return mb_split<R, d, b>(dba_mode, st, g, f, P);
     DBA_MB_SHAPES(XM)
 #undef XM
     (void)lz;
     (void)tiles;
+    (void)grid;
     return cudaErrorInvalidValue;
 }
 
