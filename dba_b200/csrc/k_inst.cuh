@@ -43,10 +43,32 @@ static int mb_prepare(int sms)
     return grid_of<R>((const void*)cons_correct<R>, 0, sms);
 }
 
+// 3-D dendrite tiles: shared-memory limit on the current device, resident CTAs
+template <typename R, int B>
+static int den3_prepare(int sms)
+{
+    using S = Den3<R, B>;
+    cudaFuncSetAttribute(dendrite3_step<R, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaFuncSetAttribute(dendrite3_step<R, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    return grid_of<R>((const void*)dendrite3_step<R, B, true>, S::smem, sms);
+}
+
+template <typename R, int B>
+static cudaError_t den3_launch(bool dba_mode, cudaStream_t st, const GridP& g, const FlagP& f, const DenP<R>& P)
+{
+    using S = Den3<R, B>;
+    const int nt = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY) * ((g.nz + S::TZ - 1) / S::TZ);
+    if (dba_mode) dendrite3_step<R, B, true><<<nt, S::NT, S::smem, st>>>(g, f, P);
+    else dendrite3_step<R, B, false><<<nt, S::NT, S::smem, st>>>(g, f, P);
+    return cudaGetLastError();
+}
+
 template <typename R>
 int step_grid(int model, int D, int B, int sms)
 {
-#define XD(d, b) if (D == d && B == b) return grid_of<R>((const void*)dendrite_step<R, d, b, true>, 0, sms);
+#define XD(d, b) if (D == d && B == b) { \
+    if constexpr (d == 3) return den3_prepare<R, b>(sms); \
+    else return grid_of<R>((const void*)dendrite_step<R, d, b, true>, 0, sms); }
 #define XM(d, b) if (D == d && B == b) { \
     if constexpr (sizeof(R) == 4 && d == 2) return grid_of<R>((const void*)modelb_fast_step<b, true>, MBFastShape<b>::smem, sms); \
     else return mb_prepare<R, d, b>(sms); }
@@ -66,8 +88,11 @@ cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, cudaStream_t 
 {
 #define XD(d, b)                                                                   \
     if (D == d && B == b) {                                                        \
-        if (dba_mode) dendrite_step<R, d, b, true><<<grid, kThreads, 0, st>>>(g, f, P); \
-        else dendrite_step<R, d, b, false><<<grid, kThreads, 0, st>>>(g, f, P);   \
+        if constexpr (d == 3) return den3_launch<R, b>(dba_mode, st, g, f, P);     \
+        else {                                                                     \
+            if (dba_mode) dendrite_step<R, d, b, true><<<grid, kThreads, 0, st>>>(g, f, P); \
+            else dendrite_step<R, d, b, false><<<grid, kThreads, 0, st>>>(g, f, P); \
+        }                                                                          \
         return cudaGetLastError();                                                 \
     }
     DBA_DEN_SHAPES(XD)

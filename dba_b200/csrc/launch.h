@@ -7,6 +7,7 @@
 
 #include "k_common.cuh"
 #include "k_dendrite.cuh"
+#include "k_dendrite3.cuh"
 #include "k_dendrite_tile.cuh"
 #include "k_kh.cuh"
 #include "k_kh_tile.cuh"
