@@ -69,68 +69,73 @@ static DBA_FM_HD double dba_fm_pow2i(int k)
     return dba_fm_from_bits((int64_t)(k + 1023) << 52);
 }
 
+/* One range test sends the ordinary arguments straight to the arithmetic; integers are
+   rounded and converted with the 1.5 2^52 and 2^52 + 2^31 offsets, whose sums are exact
+   (the conversion and rounding instructions run at a quarter of the FP64 rate). */
 static DBA_FM_HD double dba_exp(double x)
 {
-    if (x != x) return x;                       /* NaN */
-    if (x > 709.782712893384) return dba_fm_from_bits(0x7ff0000000000000LL);
-    if (x < -745.1332191019412) return 0.0;
-    double kd = rint(x * DBA_FM_INV_LN2);
+    const uint32_t ah = (uint32_t)((uint64_t)dba_fm_bits(x) >> 32) & 0x7fffffffu;
+    if (ah >= 0x40862000u) {                    /* |x| >= 708, inf, NaN */
+        if (x != x) return x;                   /* NaN */
+        if (x > 709.782712893384) return dba_fm_from_bits(0x7ff0000000000000LL);
+        if (x < -745.1332191019412) return 0.0;
+    }
+    const double t = x * DBA_FM_INV_LN2 + 6755399441055744.0;   /* 1.5 2^52 */
+    const double kd = t - 6755399441055744.0;                   /* rint(x / ln2) */
+    const int k = (int)(uint32_t)dba_fm_bits(t);       /* its low word */
     double r = fma(-kd, DBA_FM_LN2_HI, x);
     r = fma(-kd, DBA_FM_LN2_LO, r);
     double q = fma(r * r, dba_fm_exp_poly(r), r);  /* exp(r) - 1 */
     double y = 1.0 + q;
-    int k = (int)kd;
-    if (k > 1023) return (y * 2.0) * dba_fm_pow2i(k - 1);
-    if (k < -1022) return (y * dba_fm_pow2i(k + 600)) * dba_fm_pow2i(-600);
+    if (ah >= 0x40862000u) {
+        if (k > 1023) return (y * 2.0) * dba_fm_pow2i(k - 1);
+        if (k < -1022) return (y * dba_fm_pow2i(k + 600)) * dba_fm_pow2i(-600);
+    }
     return y * dba_fm_pow2i(k);
 }
 
 static DBA_FM_HD double dba_log(double x)
 {
-    if (x != x) return x;
-    if (x < 0.0) return dba_fm_from_bits(0x7ff8000000000000LL);
-    if (x == 0.0) return -dba_fm_from_bits(0x7ff0000000000000LL);
     int64_t b = dba_fm_bits(x);
-    if ((b >> 52) >= 0x7ff) return x;           /* +inf */
-    int e = 0;
-    if ((b >> 52) == 0) {                       /* subnormal */
-        x *= 18014398509481984.0;               /* 2^54 */
+    int e = -1023;
+    if ((uint32_t)((uint64_t)b >> 32) - 0x00100000u >= 0x7fe00000u) {   /* not a positive normal number */
+        if (x != x) return x;
+        if (x < 0.0) return dba_fm_from_bits(0x7ff8000000000000LL);
+        if (x == 0.0) return -dba_fm_from_bits(0x7ff0000000000000LL);
+        if ((b >> 52) >= 0x7ff) return x;       /* +inf */
+        x *= 18014398509481984.0;               /* subnormal: times 2^54 */
         b = dba_fm_bits(x);
-        e = -54;
+        e -= 54;
     }
-    e += (int)((b >> 52) & 0x7ff) - 1023;
-    double m = dba_fm_from_bits((b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-    if (m > DBA_FM_SQRT2) {
-        m *= 0.5;
+    e += (int)((uint64_t)b >> 52);
+    int64_t mb = (b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL;
+    if (mb > 0x3ff6a09e667f3bcdLL) {            /* sqrt(2): m / 2 */
+        mb -= 0x0010000000000000LL;
         e += 1;
     }
+    const double m = dba_fm_from_bits(mb);
     double f = m - 1.0;
     double s = f / (2.0 + f);
     double z = s * s;
     double lm = fma(s * z, dba_fm_log_poly(z), 2.0 * s);
-    double ed = (double)e;
+    /* (double)e */
+    const double ed = dba_fm_from_bits(0x4330000000000000LL | (int64_t)(uint32_t)((uint32_t)e + 0x80000000u)) - 4503601774854144.0;
     return fma(ed, DBA_FM_LN2_HI, fma(ed, DBA_FM_LN2_LO, lm));
 }
 
+/* The three intervals differ in the quotient t alone (t = a is the exact a / 1), so the
+   lanes of a warp share one division and one polynomial. */
 static DBA_FM_HD double dba_atan(double x)
 {
     if (x != x) return x;
-    double a = fabs(x);
-    double r;
-    if (a <= DBA_FM_TAN_PI8) {
-        double z = a * a;
-        r = fma(a * z, dba_fm_atan_poly(z), a);
-    } else if (a < DBA_FM_TAN_3PI8) {
-        double t = (a - 1.0) / (a + 1.0);
-        double z = t * t;
-        double at = fma(t * z, dba_fm_atan_poly(z), t);
-        r = DBA_FM_PIO4_HI + (at + DBA_FM_PIO4_LO);
-    } else {
-        double t = 1.0 / a;                     /* a = inf gives t = 0 */
-        double z = t * t;
-        double at = fma(t * z, dba_fm_atan_poly(z), t);
-        r = DBA_FM_PIO2_HI - (at - DBA_FM_PIO2_LO);
-    }
+    const double a = fabs(x);
+    const bool lo = a <= DBA_FM_TAN_PI8, mid = !lo && a < DBA_FM_TAN_3PI8;
+    const double num = lo ? a : (mid ? a - 1.0 : 1.0);
+    const double den = lo ? 1.0 : (mid ? a + 1.0 : a);
+    const double t = num / den;                 /* a = inf gives t = 0 */
+    const double z = t * t;
+    const double at = fma(t * z, dba_fm_atan_poly(z), t);
+    const double r = lo ? at : (mid ? DBA_FM_PIO4_HI + (at + DBA_FM_PIO4_LO) : DBA_FM_PIO2_HI - (at - DBA_FM_PIO2_LO));
     return x < 0.0 ? -r : r;
 }
 
