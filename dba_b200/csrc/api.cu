@@ -41,6 +41,7 @@ struct dba_ctx {
     int device = 0, sms = 148, grid = 148;
     cudaStream_t st = nullptr;
     std::vector<Alloc> allocs;        // every device allocation (checkpointed in order)
+    std::vector<Alloc> work;          // workspaces that carry nothing from step to step (not checkpointed)
     void* state[4][2] = {};           // ping-pong state fields (dendrite p,T; Model B x,y,z) / KH U in [q][0]
     void* aux[32] = {};               // Model B mu[3]; KH W[4] Gd[8] Wp[4] Fl[8]
     uint8_t* par = nullptr;           // [2][nch][nb]
@@ -66,6 +67,7 @@ struct dba_ctx {
     float* fstaging = nullptr;        // dba_read_field_f32: a field as floats (allocated on first use)
     bool kh_tiles = false;            // KH one-kernel step on 16x16-cell tiles (k_kh_tile.cuh)
     bool den_tiles = false;           // FP32 3-D dendrite on 32x8x8-cell tiles (k_dendrite_tile.cuh)
+    bool den3_list = false;           // 3-D dendrite through the general tile kernel: list in tlist, counts in tctr[step % 2]
     double lazy_ncells = 0;           // divisor of the FP32 conserved offset when the context is a slab of a
                                       //   larger domain (dba_slab_rows); 0: this context's cells
     int* tlist = nullptr;             // tile queue of the tile kernels that take tiles dynamically
@@ -103,6 +105,26 @@ void* dev_alloc(dba_ctx* c, size_t bytes, int* err)
     return p;
 }
 
+void* work_alloc(dba_ctx* c, size_t bytes, int* err)
+{
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaSuccess) e = cudaMemset(p, 0, bytes);
+    if (e != cudaSuccess) {
+        if (p) cudaFree(p);
+        *err = cuda_status(e);
+        return nullptr;
+    }
+    c->work.push_back({p, bytes});
+    return p;
+}
+
+// the state was replaced: no list of the step before it is valid
+int reset_work(dba_ctx* c)
+{
+    return c->den3_list ? cuda_status(cudaMemsetAsync(c->tctr, 0, 4 * sizeof(unsigned), c->st)) : DBA_OK;
+}
+
 int nfields_of(int model) { return model == DBA_MODEL_DENDRITE ? 2 : (model == DBA_MODEL_MODELB ? 7 : 8); }
 
 GridP make_grid(const dba_config& c, int B)
@@ -130,6 +152,10 @@ FlagP flags_for(dba_ctx* c, long s)
     f.stats = c->stats;
     f.tlist = c->tlist;
     f.tctr = c->tctr;
+    if (c->den3_list) {
+        f.tctr = c->tctr + s % 2;
+        f.tctr_nxt = c->tctr + (s + 1) % 2;
+    }
     return f;
 }
 
@@ -724,12 +750,24 @@ int dba_create(const dba_config* cfg, dba_ctx** out)
     }
     c->grid = c->esz == 8 ? step_grid<double>(cfg->model, c->D, c->B, c->sms) : step_grid<float>(cfg->model, c->D, c->B, c->sms);
     if (c->grid < 1) c->grid = c->sms;
-    if (cfg->model == DBA_MODEL_DENDRITE && c->esz == 4 && cfg->tiles && dendrite_tiles_ok(c->D, c->B, cfg->nx, cfg->ny, cfg->nz)) {
-        const size_t nt = (size_t)(cfg->nx / 32) * (cfg->ny / 8) * (cfg->nz / 8);
-        c->den_tiles = true;
-        c->grid = dendrite3_tile_grid(c->sms, (int)nt);
-        c->tlist = (int*)dev_alloc(c, 2 * nt * sizeof(int), &err);
-        if (!err) c->tctr = (unsigned*)dev_alloc(c, 4 * sizeof(unsigned), &err);
+    if (cfg->model == DBA_MODEL_DENDRITE && c->D == 3) {
+        const int nt = dendrite3_tiles(cfg->nx, cfg->ny, cfg->nz);
+        const bool listed = dendrite3_listed(nt, c->grid);
+        const bool dbuf = c->esz == 4 && cfg->tiles && dendrite_tiles_ok(c->D, c->B, cfg->nx, cfg->ny, cfg->nz);
+        if (dbuf && (listed || cfg->nx % 32 == 0)) {
+            // (checkpoints of FP32 grids of whole tiles hold the list, used or not; it is empty between steps)
+            auto alloc = cfg->nx % 32 == 0 ? dev_alloc : work_alloc;
+            c->tlist = (int*)alloc(c, 2 * (size_t)nt * sizeof(int), &err);
+            if (!err) c->tctr = (unsigned*)alloc(c, 4 * sizeof(unsigned), &err);
+        }
+        if (dbuf && listed) {
+            c->den_tiles = true;
+            c->grid = dendrite3_tile_grid(c->sms, nt);
+        } else if (listed) {
+            c->den3_list = true;
+            c->tlist = (int*)work_alloc(c, (size_t)nt * kDen3Entry * sizeof(int), &err);
+            if (!err) c->tctr = (unsigned*)work_alloc(c, 4 * sizeof(unsigned), &err);
+        }
         if (err) {
             dba_destroy(c);
             return err;
@@ -776,6 +814,7 @@ void dba_destroy(dba_ctx* c)
             for (auto& gexec : row)
                 if (gexec) cudaGraphExecDestroy(gexec);
     for (auto& a : c->allocs) cudaFree(a.p);
+    for (auto& a : c->work) cudaFree(a.p);
     if (c->fstaging) cudaFree(c->fstaging);
     if (c->host_staging) cudaFreeHost(c->host_staging);
     if (c->st) cudaStreamDestroy(c->st);
@@ -843,7 +882,7 @@ int dba_init(dba_ctx* c, const double* ic)
     c->step = 0;
     c->time = 0.0;
     c->initialized = true;
-    return DBA_OK;
+    return reset_work(c);
 }
 
 int dba_init_f32(dba_ctx* c, const float* ic)
@@ -870,7 +909,7 @@ int dba_init_f32(dba_ctx* c, const float* ic)
     c->step = 0;
     c->time = 0.0;
     c->initialized = true;
-    return DBA_OK;
+    return reset_work(c);
 }
 
 int dba_step(dba_ctx* c, int nsteps, int mode)
@@ -1251,6 +1290,7 @@ int dba_get_info(dba_ctx* c, dba_info* info)
     info->nchannels = c->nch;
     size_t bytes = 0;
     for (auto& a : c->allocs) bytes += a.bytes;
+    for (auto& a : c->work) bytes += a.bytes;
     info->device_bytes = bytes;
     info->step = c->step;
     info->grid_ctas = c->grid;
@@ -1404,7 +1444,7 @@ int dba_load_state(dba_ctx* c, const void* host, size_t size)
         off += a.bytes;
     }
     c->initialized = true;
-    return DBA_OK;
+    return reset_work(c);
 }
 
 int dba_get_config(dba_ctx* c, dba_config* cfg)
@@ -1474,7 +1514,7 @@ int dba_restore(dba_ctx* c, const char* path)
     c->step = step;
     c->time = time;
     c->initialized = true;
-    return DBA_OK;
+    return reset_work(c);
 }
 
 int dba_tip_profile(dba_ctx* c, int field, int dz, int* tip_x, int* tip_x_max)

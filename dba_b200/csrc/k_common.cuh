@@ -51,6 +51,7 @@ struct FlagP {
     // (tile_list_append / tile_queue_done); null elsewhere
     int* tlist = nullptr;       // (tile, meta) pairs
     unsigned* tctr = nullptr;   // [0] entries listed, [1] entries taken, [2] CTAs done
+    unsigned* tctr_nxt = nullptr;   // k_dendrite3.cuh: tctr is this step's count alone, this the next step's
 };
 
 __device__ __forceinline__ int wrapc(int v, int n, int bc)

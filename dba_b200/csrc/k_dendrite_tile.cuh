@@ -59,16 +59,18 @@ __global__ void __launch_bounds__(256) dendrite3_tile_scan(GridP g, FlagP f)
 {
     constexpr int B = DenTile::B, TX = DenTile::TX, TBX = DenTile::TBX;
     const int nb = g.nb;
-    const int ntx = g.nx / TX, nty = g.ny / B, ntz = g.nz / B;
+    const int ntx = (g.nx + TX - 1) / TX, nty = g.ny / B, ntz = g.nz / B;
     const long long nitems = (long long)ntx * nty * ntz * TBX;
     for (long long t0 = (long long)blockIdx.x * blockDim.x; t0 < nitems; t0 += (long long)gridDim.x * blockDim.x) {
         const long long it = t0 + threadIdx.x;
-        const bool valid = it < nitems;
         const int tile = (int)(it / TBX), kq = (int)(it % TBX);
-        int act = 0, pp = 0, pT = 0, entry = 0;
+        const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
+        const int entry = tx | (ty << 10) | (tz << 20);
+        // the last tile of a row may reach past the grid: its blocks there are never active, so
+        // no piece beyond the last block's halo is staged
+        const bool valid = it < nitems && tx * TBX + kq < g.nbx;
+        int act = 0, pp = 0, pT = 0;
         if (valid) {
-            const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
-            entry = tx | (ty << 10) | (tz << 20);
             const int b = (tx * TBX + kq) + g.nbx * (ty + g.nby * tz);
             pp = f.par_cur[b];
             pT = f.par_cur[nb + b];
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
 
     const int tid = threadIdx.x;
     const int nb = g.nb;
-    const int ntx = g.nx / TX, nty = g.ny / B;
+    const int ntx = (g.nx + TX - 1) / TX, nty = g.ny / B;
     const size_t nx = (size_t)g.nx, nxy = (size_t)g.nx * g.ny;
     const DenC32 C = P.c32;
     const float dt = (float)P.dt;
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
             if (gx0 >= 0 && gx0 + 3 < g.nx) {
                 cp_async16(dst + so, pb + row + gx0);
                 cp_async16(dst + SV + so, Tb + row + gx0);
-            } else if (!g.bc) {                    // periodic: the piece wraps whole (nx is a multiple of 32)
+            } else if (!g.bc) {                    // periodic: the piece wraps whole (nx is a multiple of 8)
                 const int gx = gx0 < 0 ? gx0 + g.nx : gx0 - g.nx;
                 cp_async16(dst + so, pb + row + gx);
                 cp_async16(dst + SV + so, Tb + row + gx);

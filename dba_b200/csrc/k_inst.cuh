@@ -48,18 +48,37 @@ template <typename R, int B>
 static int den3_prepare(int sms)
 {
     using S = Den3<R, B>;
-    cudaFuncSetAttribute(dendrite3_step<R, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
-    cudaFuncSetAttribute(dendrite3_step<R, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
-    return grid_of<R>((const void*)dendrite3_step<R, B, true>, S::smem, sms);
+    cudaFuncSetAttribute(dendrite3_step<R, B, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaFuncSetAttribute(dendrite3_step<R, B, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaFuncSetAttribute(dendrite3_step<R, B, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaFuncSetAttribute(dendrite3_step<R, B, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    return grid_of<R>((const void*)dendrite3_step<R, B, true, true>, S::smem, sms);
 }
 
+// the scan lists the step's tiles and the tile kernel steps through the list, or, on a small
+// grid, one CTA per tile reads its own flags
 template <typename R, int B>
-static cudaError_t den3_launch(bool dba_mode, cudaStream_t st, const GridP& g, const FlagP& f, const DenP<R>& P)
+static cudaError_t den3_launch(bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f, const DenP<R>& P)
 {
     using S = Den3<R, B>;
-    const int nt = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY) * ((g.nz + S::TZ - 1) / S::TZ);
-    if (dba_mode) dendrite3_step<R, B, true><<<nt, S::NT, S::smem, st>>>(g, f, P);
-    else dendrite3_step<R, B, false><<<nt, S::NT, S::smem, st>>>(g, f, P);
+    const int nt = dendrite3_tiles(g.nx, g.ny, g.nz);
+    if (!dendrite3_listed(nt, grid)) {
+        if (dba_mode) dendrite3_step<R, B, true, false><<<nt, S::NT, S::smem, st>>>(g, f, P, nt);
+        else dendrite3_step<R, B, false, false><<<nt, S::NT, S::smem, st>>>(g, f, P, nt);
+        return cudaGetLastError();
+    }
+    // 8 times as many CTAs as are resident: fewer listed tiles than that (most DBA steps) get
+    // one CTA each, and an unused CTA ends after reading the count
+    if (!f.tlist || !f.tctr || !f.tctr_nxt) return cudaErrorInvalidValue;
+    const int ng = 8 * grid < nt ? 8 * grid : nt;
+    const int sg = (int)(((long long)nt * S::NBT + 255) / 256);
+    if (dba_mode) {
+        dendrite3_scan<R, B, true><<<sg, 256, 0, st>>>(g, f, nt);
+        dendrite3_step<R, B, true, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
+    } else {
+        dendrite3_scan<R, B, false><<<sg, 256, 0, st>>>(g, f, nt);
+        dendrite3_step<R, B, false, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
+    }
     return cudaGetLastError();
 }
 
@@ -88,7 +107,7 @@ cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, cudaStream_t 
 {
 #define XD(d, b)                                                                   \
     if (D == d && B == b) {                                                        \
-        if constexpr (d == 3) return den3_launch<R, b>(dba_mode, st, g, f, P);     \
+        if constexpr (d == 3) return den3_launch<R, b>(dba_mode, grid, st, g, f, P); \
         else {                                                                     \
             if (dba_mode) dendrite_step<R, d, b, true><<<grid, kThreads, 0, st>>>(g, f, P); \
             else dendrite_step<R, d, b, false><<<grid, kThreads, 0, st>>>(g, f, P); \

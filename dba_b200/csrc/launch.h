@@ -27,13 +27,24 @@ template <typename R> int step_grid(int model, int D, int B, int sms);
 template <typename R>
 cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                             const DenP<R>& P);
-// FP32 3-D dendrite on 32x8x8-cell tiles (k_dendrite_tile.cuh)
+// FP32 3-D dendrite on double-buffered 32x8x8-cell tiles (k_dendrite_tile.cuh), for grids that
+// need a tile list (dendrite3_listed)
 // (tile coordinates are packed into 10-bit fields of the tile-queue entry)
 inline bool dendrite_tiles_ok(int D, int B, int nx, int ny, int nz)
 {
-    return D == 3 && B == 8 && nx % 32 == 0 && nx / 32 <= 1024 && ny / 8 <= 1024 && nz / 8 <= 1024;
+    return D == 3 && B == 8 && (nx + 31) / 32 <= 1024 && ny / 8 <= 1024 && nz / 8 <= 1024;
 }
 int dendrite3_tile_grid(int sms, int ntiles);
+// tiles of the general 3-D dendrite kernel (k_dendrite3.cuh)
+inline int dendrite3_tiles(int nx, int ny, int nz) { return ((nx + 31) / 32) * ((ny + 7) / 8) * ((nz + 7) / 8); }
+// Whether it works from a list (resident: CTAs on the GPU at once).  The scan is a launch of
+// its own, about 3 us; without it each idle tile costs a CTA that reads its flags and ends.
+// us per step, list / none: FP64 4^3 blocks 128^3 (2.3 tiles per resident CTA) 30.4 / 26.9,
+// 192x160x96 (3.2) 26.9 / 25.1, 256^3 (18) 67.7 / 76.7; FP32 8^3 200x136x104 (2.1)
+// 19.5 / 17.0, 256^3 (11) 31.7 / 38.0.
+// FP32 8^3 grids that need a list take the double-buffered tiles of k_dendrite_tile.cuh instead:
+// 512^3 dense 745 against 779 us, 256^3 106 against 107, but 200x136x104 29.6 against 25.1.
+inline bool dendrite3_listed(int tiles, int resident) { return tiles > 4 * resident; }
 cudaError_t launch_dendrite3_tiles(bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                                    const DenP<float>& P);
 // FP32 2-D uses the fast kernels (lazy conserved correction, reduction fused):

@@ -25,13 +25,14 @@ def _seed(nx, ny, nz, r):
 @pytest.mark.parametrize("nx,ny,nz,B,mode,bc,precision", [
     (36, 20, 12, 4, 1, 0, 0), (36, 20, 12, 4, 1, 1, 0), (40, 24, 16, 8, 1, 0, 0), (72, 24, 8, 8, 1, 1, 0),
     (4, 4, 4, 4, 1, 0, 0), (8, 8, 8, 8, 1, 1, 0), (68, 12, 20, 4, 0, 1, 0), (40, 16, 24, 8, 0, 0, 0),
-    (36, 20, 12, 4, 1, 1, 1), (68, 12, 20, 4, 0, 0, 1), (40, 24, 16, 8, 1, 1, 1)])
+    (36, 20, 12, 4, 1, 1, 1), (68, 12, 20, 4, 0, 0, 1), (40, 24, 16, 8, 1, 1, 1), (200, 128, 144, 4, 1, 0, 0),
+    (136, 144, 168, 8, 1, 1, 0)])                       # the last two work from a tile list
 def test_dendrite3_tile_edges(nx, ny, nz, B, mode, bc, precision):
-    p, T = _seed(nx, ny, nz, 3.0)
+    p, T = _seed(nx, ny, nz, 3.0 if nx < 100 else 12.0)
     o = OracleDendrite(nx, ny, nz, B, DEN, bc=bc)
     o.set_fields(p, T)
     s = dba_b200.Simulation(dendrite_cfg(DEN, nx, ny, nz, B, precision=precision, bc=bc)).init([p, T])
-    for t in range(1, 31):
+    for t in range(1, 31 if nx < 100 else 9):
         o.step(1, mode)
         s.step(1, mode)
         if precision:
@@ -45,6 +46,23 @@ def test_dendrite3_tile_edges(nx, ny, nz, B, mode, bc, precision):
     d = o.get()
     assert np.max(np.abs(s.field("p") - d["p"])) <= 2e-5 and np.max(np.abs(s.field("T") - d["T"])) <= 2e-5
     s.sync()
+
+
+@pytest.mark.parametrize("nx,ny,nz,bc", [(200, 256, 256, 0), (136, 256, 256, 1), (256, 256, 128, 1)])
+def test_dendrite3_fp32_tiles_past_the_grid(nx, ny, nz, bc):
+    """FP32 8^3 blocks on grids that work from a tile list: the double-buffered tiles, whose last
+    tile of a row may reach past the grid, equal the general tile kernel bit for bit."""
+    p, T = _seed(nx, ny, nz, 20.0)
+    a, b = (dba_b200.Simulation(dendrite_cfg(DEN, nx, ny, nz, 8, precision=1, bc=bc, tiles=t)).init([p, T]) for t in (1, 0))
+    for n, mode in ((1, 1), (1, 1), (30, 1), (3, 0), (40, 1)):
+        for s in (a, b):
+            s.step(n, mode)
+        for q in ("p", "T"):
+            assert np.array_equal(a.field(q), b.field(q)), (q, n)
+        for w in range(4):
+            assert np.array_equal(a.flags(w), b.flags(w)), (w, n)
+    a.sync()
+    b.sync()
 
 
 @pytest.mark.parametrize("nx,ny,nz,B,mode,conserved,precision", [
