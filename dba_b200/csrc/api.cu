@@ -900,7 +900,11 @@ int dba_init_f32(dba_ctx* c, const float* ic)
     // ordered on the context's stream like the copies: a clear on the default stream does not
     // wait for the stream and may still run when the first copy writes the field it clears
     DBA_TRY(cudaStreamSynchronize(c->st));
-    for (auto& a : c->allocs) DBA_TRY(cudaMemsetAsync(a.p, 0, a.bytes, c->st));
+    for (auto& a : c->allocs) {
+        bool written = a.p == (void*)c->staging;          // scratch, or written whole by the copies below
+        for (int q = 0; q < c->nstate; ++q) written |= a.p == c->state[q][0];
+        if (!written) DBA_TRY(cudaMemsetAsync(a.p, 0, a.bytes, c->st));
+    }
     for (int q = 0; q < c->nstate; ++q)
         DBA_TRY(cudaMemcpyAsync(c->state[q][0], ic + q * c->n, c->n * sizeof(float), cudaMemcpyHostToDevice, c->st));
     // step 1 reads wake[1 % 3]: every block starts active (as dba_init)
