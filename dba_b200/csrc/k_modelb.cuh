@@ -29,11 +29,15 @@
 // cell of traffic and computes each once; a single kernel that recomputed them on every
 // block's halo (the form before) did 3.4 times the potential work at 4^3 blocks and
 // staged 8 cells for each that it advanced.
-// A thread owns 4 cells along z and walks down the planes, one field after the other; a
-// cell's sums take each plane's values as it arrives (LapZ), so a value is loaded 9 to
-// 14 times, not 27, and 16 registers carry what a window of three planes would need 54 for.
-// Measured per step, every block active: 256^3 FP64 in 4^3 blocks 5.17 -> 0.85 ms, 192^3 FP32
-// in 8^3 blocks (regular) 0.554 -> 0.222 ms, 768^2 FP64 conserved in 16^2 blocks 69 -> 58 us.
+// A thread owns 4 cells along z (8 in FP32 8^3 blocks) and walks down the planes, one field
+// after the other; a cell's sums take each plane's values as it arrives (LapZ), so a value
+// is loaded 9 to 14 times, not 27, and 16 registers carry what a window of three planes
+// would need 54 for.  The pointwise part is one copy of the code per kernel (unrolled
+// over the cells, its logarithms and exponentials overflowed the instruction cache), and
+// 64 registers leave four CTAs per SM: 3 CTAs at 80 registers took 792 us where 4 take 708.
+// Measured per step, every block active, before -> now: 256^3 FP64 in 4^3 blocks 5167 ->
+// 708 us, 192^3 FP32 in 8^3 blocks (regular) 554 -> 168 us, 4^3 blocks 1088 -> 187 us;
+// 768^2 FP64 in 4^2 blocks 72.9 -> 34.2 us, conserved in 16^2 blocks 69 -> 54 us.
 // The Nz == 1 form keeps the reference's 27-term sum with the z neighbours
 // wrapped onto the cell itself.
 #pragma once
@@ -121,8 +125,9 @@ struct LapZ {
 };
 
 // Tile shapes: 3-D 32 x 8 x 4 (4^3 blocks), 16 x 8 x 8 (8^3, FP64), 32 x 8 x 8 (8^3, FP32):
-// a tile holds whole blocks, and the staged box of three fields leaves room for 4 CTAs
-// (modelb_mu at 32 x 8 x 8 in FP64: 86 KB, 2 CTAs, and half the speed).
+// a tile holds whole blocks, and the staged box of three fields leaves room for 4 CTAs of
+// 256 threads (modelb_mu at 32 x 8 x 8 in FP64: 86 KB, 2 CTAs, and half the speed; FP32 8^3
+// with 4 cells per thread and CTAs of 512: 223 us where 8 cells and 256 threads take 168).
 template <typename R, int D, int B>
 struct MBShape {
     static constexpr int TX = D == 3 && B == 8 && sizeof(R) == 8 ? 16 : 32;
@@ -132,15 +137,15 @@ struct MBShape {
     static constexpr int PC = 16 / (int)sizeof(R);       // cells per staged piece (B is a multiple)
     static constexpr int SW = TX + 2 * PC, SH = TY + 2, SD = D == 3 ? TZ + 2 : 1;           // staged box
     static constexpr int PL = SW * SH, SV = PL * SD;     // one staged plane, one staged field
-    static constexpr int NPR = SW / PC, NPF = NPR * SH * SD;
-    static constexpr int NC = D == 3 ? 4 : TY / 8;       // cells per thread: along z, in 2-D along y
+    static constexpr int NPR = SW / PC;                  // pieces per staged row
+    static constexpr int NC = D == 3 ? (sizeof(R) == 4 ? B : 4) : TY / 8;       // cells per thread: along z, in 2-D along y
     static constexpr int CELLS = TX * TY * TZ, NT = CELLS / NC;
-    static constexpr int MINB = 1024 / NT - (sizeof(R) == 8 ? 1 : 0);   // resident CTAs per SM: 80 registers in FP64, 64 in FP32
+    static constexpr int MINB = 1024 / NT;               // resident CTAs per SM: 64 registers per thread
     static constexpr size_t smem_mu = sizeof(R) * 3 * SV;
     static constexpr size_t smem_chg = sizeof(double) * 3 * CELLS;      // modelb_update, conserved: the cells' changes,
     static constexpr size_t smem_cons = smem_mu > smem_chg ? smem_mu : smem_chg;   // in the staged potentials' place
     static_assert(NBT <= 32 && NBT >= 1 && B % PC == 0 && TX % B == 0 && TY % B == 0, "a tile's blocks fit one warp");
-    static_assert((NT == 256 || NT == 512) && (D == 3 ? B % NC == 0 : B % NC == 0), "a thread's cells lie in one block");
+    static_assert(NT == 256 && B % NC == 0, "a thread's cells lie in one block");
     // first cell (x, y, z) of thread tid
     static __device__ __forceinline__ void first(int tid, int& x, int& y, int& z)
     {
@@ -213,6 +218,33 @@ __device__ __forceinline__ void tile_block_sums(const double* s_val, unsigned ma
         }
         if (lane == 0) s_out[k] = out;
     }
+}
+
+// The 16-byte pieces of the tile's part inside the grid and one cell around it: a thread
+// keeps one piece of a plane (so its column, row and wrap are worked out once) and steps
+// over the planes.  body(cell index, staged offset, index in the table of blocks).
+template <typename S, int D, int B, typename T, typename F>
+__device__ __forceinline__ void stage_pieces(const GridP& g, const T& t, F&& body)
+{
+    constexpr int PP = S::NPR * S::SH, ZP = PP <= S::NT ? S::NT / PP : 1;   // pieces of a plane; planes at once
+    const int ph = PP <= S::NT ? (int)threadIdx.x / PP : 0;
+    if (ph >= ZP) return;
+    for (int i = (int)threadIdx.x - ph * PP; i < PP; i += PP <= S::NT ? PP : S::NT) {
+        const int c = i % S::NPR, ry = i / S::NPR;
+        const int lx = (c - 1) * S::PC, ly = ry - 1;
+        if (lx > t.vx || ly > t.vy) continue;
+        const int reg = (lx + B) / B + S::RX * ((ly + B) / B);
+        const size_t row = (size_t)wrap_p(t.X0 + lx, g.nx) + (size_t)g.nx * wrap_p(t.Y0 + ly, g.ny);
+        if constexpr (D == 3) {
+            const size_t nxy = (size_t)g.nx * g.ny;
+#pragma unroll 2
+            for (int rz = ph; rz < S::SD && rz - 1 <= t.vz; rz += ZP)
+                body(row + nxy * wrap_p(t.Z0 + rz - 1, g.nz), rz * S::PL + i * S::PC, reg + S::RX * S::RY * ((rz - 1 + B) / B));
+        } else {
+            body(row, i * S::PC, reg);
+        }
+    }
+    cp_async_commit();
 }
 
 // Laplacians of a thread's NC cells from a staged field; s = the thread's first cell
@@ -296,21 +328,12 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     const unsigned fresh = s_fresh, own = s_own;
     if (fresh == 0) return;
 
-    // x, y, z of the tile's part inside the grid and one cell around it
-    for (int i = tid; i < S::NPF; i += NT) {
-        const int c = i % S::NPR, ry = (i / S::NPR) % S::SH, rz = i / (S::NPR * S::SH);
-        const int lx = (c - 1) * S::PC, ly = ry - 1, lz = D == 3 ? rz - 1 : 0;
-        if (lx > t.vx || ly > t.vy || (D == 3 && lz > t.vz)) continue;
-        const int reg = (lx + B) / B + S::RX * ((ly + B) / B + (D == 3 ? S::RY * ((lz + B) / B) : 0));
-        const int gx = wrap_p(t.X0 + lx, g.nx), gy = wrap_p(t.Y0 + ly, g.ny), gz = D == 3 ? wrap_p(t.Z0 + lz, g.nz) : 0;
-        const size_t gi = (size_t)gx + (size_t)g.nx * ((size_t)gy + (size_t)g.ny * gz);
+    stage_pieces<S, D, B>(g, t, [&](size_t gi, int so, int reg) {
         const int par = s_tab[reg];
-        R* d = stage + (size_t)i * S::PC;
-        cp_async16(d, (par ? P.x[1] : P.x[0]) + gi);
-        cp_async16(d + SV, (par ? P.y[1] : P.y[0]) + gi);
-        cp_async16(d + 2 * SV, (par ? P.z[1] : P.z[0]) + gi);
-    }
-    cp_async_commit();
+        cp_async16(stage + so, (par ? P.x[1] : P.x[0]) + gi);
+        cp_async16(stage + SV + so, (par ? P.y[1] : P.y[0]) + gi);
+        cp_async16(stage + 2 * SV + so, (par ? P.z[1] : P.z[0]) + gi);
+    });
     cp_async_wait0();
     __syncthreads();
 
@@ -320,34 +343,39 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     const R* s0 = stage + (cy + 1) * SW + cx + S::PC + (D == 3 ? (cz + 1) * PL : 0);
     const int k = cx / B + S::NBX * (cy / B + S::NBY * (cz / B));   // the thread's block
     if ((fresh >> k) & 1u) {
-    R lap[3][NC];
+        R lap[3][NC];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) column_laps<S, R, D>(s0 + q * SV, inv_dx2, lap[q]);
-    // potentials (Calc_mu, kernel.cu:371-388)
-    auto over = [](R v, double r, double ir) { return ir != 0.0 ? v * (R)ir : v / (R)r; };
-    bool hit = false;
-    const size_t g0 = (size_t)(t.X0 + cx) + (size_t)g.nx * ((size_t)(t.Y0 + cy) + (size_t)g.ny * (t.Z0 + cz));
+        for (int q = 0; q < 3; ++q) column_laps<S, R, D>(s0 + q * SV, inv_dx2, lap[q]);
+        // potentials (Calc_mu, kernel.cu:371-388)
+        auto over = [](R v, double r, double ir) { return ir != 0.0 ? v * (R)ir : v / (R)r; };
+        bool hit = false;
+        const size_t g0 = (size_t)(t.X0 + cx) + (size_t)g.nx * ((size_t)(t.Y0 + cy) + (size_t)g.ny * (t.Z0 + cz));
+        // one copy of the code (4 logarithms a cell): the Laplacians shift down instead
+#pragma unroll 1
+        for (int c = 0; c < NC; ++c) {
+            const R* s = s0 + c * (D == 3 ? PL : SW);
+            const R X = s[0], Y = s[SV], Z = s[2 * SV];
+            const R lapx = lap[0][0], lapy = lap[1][0], lapz = lap[2][0];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const R* s = s0 + c * (D == 3 ? PL : SW);
-        const R X = s[0], Y = s[SV], Z = s[2 * SV];
-        const R lapx = lap[0][c], lapy = lap[1][c], lapz = lap[2][c];
-        const R bb = (R)1.0 - X - Y - Z;
-        const R lb = log_r<R>(bb);
-        const R ux = (R)P.c0x + (R)P.chi_xy * Y + (R)P.chi_xz * Z + (R)P.chi_xb * bb - (R)P.chi_xb * X -
-                     (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(X), P.rx, P.irx) - lb - (R)P.ex * lapx;
-        const R uy = (R)P.c0y + (R)P.chi_xy * X + (R)P.chi_yz * Z + (R)P.chi_yb * bb - (R)P.chi_xb * X -
-                     (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(Y), P.ry, P.iry) - lb - (R)P.ey * lapy;
-        const R uz = (R)P.c0z + (R)P.chi_xz * X + (R)P.chi_yz * Y + (R)P.chi_zb * bb - (R)P.chi_xb * X -
-                     (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(Z), P.rz, P.irz) - lb - (R)P.phi_term -
-                     (R)P.ez * lapz - (R)P.logK_rz;
-        const size_t gi = g0 + c * (size_t)g.nx * (D == 3 ? g.ny : 1);
-        P.mu[0][gi] = ux;
-        P.mu[1][gi] = uy;
-        P.mu[2][gi] = uz;
-        hit |= fabs(lapz) > (R)P.thr;                    // Wakeup_Next :697
-    }
-    if (DBA && hit) s_nx[k] = 1;
+            for (int q = 0; q < 3; ++q)
+#pragma unroll
+                for (int j = 0; j + 1 < NC; ++j) lap[q][j] = lap[q][j + 1];
+            const R bb = (R)1.0 - X - Y - Z;
+            const R lb = log_r<R>(bb);
+            const R ux = (R)P.c0x + (R)P.chi_xy * Y + (R)P.chi_xz * Z + (R)P.chi_xb * bb - (R)P.chi_xb * X -
+                         (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(X), P.rx, P.irx) - lb - (R)P.ex * lapx;
+            const R uy = (R)P.c0y + (R)P.chi_xy * X + (R)P.chi_yz * Z + (R)P.chi_yb * bb - (R)P.chi_xb * X -
+                         (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(Y), P.ry, P.iry) - lb - (R)P.ey * lapy;
+            const R uz = (R)P.c0z + (R)P.chi_xz * X + (R)P.chi_yz * Y + (R)P.chi_zb * bb - (R)P.chi_xb * X -
+                         (R)P.chi_yb * Y - (R)P.chi_zb * Z + over(log_r<R>(Z), P.rz, P.irz) - lb - (R)P.phi_term -
+                         (R)P.ez * lapz - (R)P.logK_rz;
+            const size_t gi = g0 + c * (size_t)g.nx * (D == 3 ? g.ny : 1);
+            P.mu[0][gi] = ux;
+            P.mu[1][gi] = uy;
+            P.mu[2][gi] = uz;
+            hit |= fabs(lapz) > (R)P.thr;                    // Wakeup_Next :697
+        }
+        if (DBA && hit) s_nx[k] = 1;
     }
     if (!DBA) return;
     __syncthreads();
@@ -367,7 +395,7 @@ template <typename R, int D, int B, bool DBA>
 __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MINB)) modelb_update(GridP g, FlagP f, MBP<R> P)
 {
     using S = MBShape<R, D, B>;
-    constexpr int NC = S::NC, SW = S::SW, PL = S::PL, SV = S::SV, NT = S::NT;
+    constexpr int NC = S::NC, SW = S::SW, PL = S::PL, SV = S::SV;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* stage = reinterpret_cast<R*>(smem_raw);           // [x, y, z potentials][SD][SH][SW]
     __shared__ unsigned s_own, s_par;
@@ -392,18 +420,10 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     const unsigned own = s_own, par = s_par;
     if (own == 0) return;
 
-    // the potentials of the tile's part inside the grid and one cell around it
-    for (int i = tid; i < S::NPF; i += NT) {
-        const int c = i % S::NPR, ry = (i / S::NPR) % S::SH, rz = i / (S::NPR * S::SH);
-        const int lx = (c - 1) * S::PC, ly = ry - 1, lz = D == 3 ? rz - 1 : 0;
-        if (lx > t.vx || ly > t.vy || (D == 3 && lz > t.vz)) continue;
-        const int gx = wrap_p(t.X0 + lx, g.nx), gy = wrap_p(t.Y0 + ly, g.ny), gz = D == 3 ? wrap_p(t.Z0 + lz, g.nz) : 0;
-        const size_t gi = (size_t)gx + (size_t)g.nx * ((size_t)gy + (size_t)g.ny * gz);
-        R* d = stage + (size_t)i * S::PC;
+    stage_pieces<S, D, B>(g, t, [&](size_t gi, int so, int) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) cp_async16(d + q * SV, P.mu[q] + gi);
-    }
-    cp_async_commit();
+        for (int q = 0; q < 3; ++q) cp_async16(stage + q * SV + so, P.mu[q] + gi);
+    });
 
     const R inv_dx2 = (R)P.inv_dx2;
     int cx, cy, cz;
@@ -416,30 +436,33 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     const int src = (par >> k) & 1u;
     cp_async_wait0();
     __syncthreads();
-    double chg[3][NC];
+    R lap[3][NC];                                        // Laplacians, then (conserved) the changes
     if (on) {
-        R lap[3][NC];
 #pragma unroll
         for (int q = 0; q < 3; ++q) column_laps<S, R, D>(s0 + q * SV, inv_dx2, lap[q]);
-        // update (Update, kernel.cu:419-434; Conserved/kernel.cu:428-440)
-#pragma unroll
+        // update (Update, kernel.cu:419-434; Conserved/kernel.cu:428-440); one copy of the code:
+        // the Laplacians shift down and the changes follow them
+#pragma unroll 1
         for (int c = 0; c < NC; ++c) {
             const R* sc = s0 + c * (D == 3 ? PL : SW);
             const R mx = sc[0], my = sc[SV], mz = sc[2 * SV];
             const size_t gi = g0 + c * gs;
             const R X = (src ? P.x[1] : P.x[0])[gi], Y = (src ? P.y[1] : P.y[0])[gi], Z = (src ? P.z[1] : P.z[0])[gi];
             const R Rr = (R)P.k0 * (exp_r<R>((R)P.nvx * mx + (R)P.mvy * my) - exp_r<R>((R)P.dvz * mz));
-            const R chx = (R)P.dtvx * ((R)P.Mx * lap[0][c] - (R)P.dn * Rr);
-            const R chy = (R)P.dtvy * ((R)P.My * lap[1][c] - (R)P.dm * Rr);
-            const R chz = (R)P.dtvz * ((R)P.Mz * lap[2][c] + Rr);
+            const R chx = (R)P.dtvx * ((R)P.Mx * lap[0][0] - (R)P.dn * Rr);
+            const R chy = (R)P.dtvy * ((R)P.My * lap[1][0] - (R)P.dm * Rr);
+            const R chz = (R)P.dtvz * ((R)P.Mz * lap[2][0] + Rr);
             const R xn = X + chx, yn = Y + chy, zn = Z + chz;
             (src ? P.x[0] : P.x[1])[gi] = xn;
             (src ? P.y[0] : P.y[1])[gi] = yn;
             (src ? P.z[0] : P.z[1])[gi] = zn;
             if (!isfinite(xn) || !isfinite(yn) || !isfinite(zn)) raise_status(f.status, 5);
-            chg[0][c] = (double)chx;
-            chg[1][c] = (double)chy;
-            chg[2][c] = (double)chz;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+#pragma unroll
+                for (int j = 0; j + 1 < NC; ++j) lap[q][j] = lap[q][j + 1];
+                lap[q][NC - 1] = q == 0 ? chx : (q == 1 ? chy : chz);
+            }
         }
     }
     if (!P.conserved) return;
@@ -451,7 +474,7 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
         for (int c = 0; c < NC; ++c)
 #pragma unroll
             for (int q = 0; q < 3; ++q)
-                s_chg[q * S::CELLS + cx + S::TX * (D == 3 ? cy + S::TY * (cz + c) : cy + c)] = chg[q][c];
+                s_chg[q * S::CELLS + cx + S::TX * (D == 3 ? cy + S::TY * (cz + c) : cy + c)] = (double)lap[q][c];
     }
     __syncthreads();
 #pragma unroll
