@@ -72,6 +72,8 @@ struct dba_ctx {
                                       //   larger domain (dba_slab_rows); 0: this context's cells
     int* tlist = nullptr;             // tile queue of the tile kernels that take tiles dynamically
     unsigned* tctr = nullptr;         //   (2 ints per tile; counters, zeroed by each step's last CTA)
+    uint8_t *kh_full = nullptr, *kh_hit = nullptr;   // KH strips (k_kh_strip.cuh): per tile, per block
+    unsigned* kh_cnt = nullptr;       //   [3] full tiles of a step, rotating
     float* kvmax = nullptr;           // KH tiles: per-block largest signal speed (CFL)
     unsigned* kgmax = nullptr;        // KH tiles: rotating maxima of the CFL speed, float bits [3]
     double* ktime = nullptr;          // KH tiles: simulated time accumulated on the device (CFL)
@@ -119,9 +121,10 @@ void* work_alloc(dba_ctx* c, size_t bytes, int* err)
     return p;
 }
 
-// the state was replaced: no list of the step before it is valid
+// the state was replaced: no list or count of the step before it is valid
 int reset_work(dba_ctx* c)
 {
+    if (c->kh_cnt) DBA_TRY(cudaMemsetAsync(c->kh_cnt, 0xff, 3 * sizeof(unsigned), c->st));
     return c->den3_list ? cuda_status(cudaMemsetAsync(c->tctr, 0, 4 * sizeof(unsigned), c->st)) : DBA_OK;
 }
 
@@ -258,6 +261,13 @@ KHTileP<R> kh_tile_params(dba_ctx* c, bool dba_mode, long s)
     P.gmax_clear = c->kgmax + (s + 1) % 3;
     P.time = c->ktime;
     P.Kc = kh_consts<R>(k.dt, P.dx, P.dy, P.vol, P.gamma);
+    if (c->kh_full && !P.conserved) {   // (the conserved step's per-block sums live in the tile kernel)
+        P.full = c->kh_full;
+        P.hit = c->kh_hit;
+        P.cnt_prev = c->kh_cnt + (s + 2) % 3;
+        P.cnt_cur = c->kh_cnt + s % 3;
+        P.cnt_next = c->kh_cnt + (s + 1) % 3;
+    }
     return P;
 }
 
@@ -778,6 +788,11 @@ int dba_create(const dba_config* cfg, dba_ctx** out)
         c->grid = c->esz == 8 ? kh_tile_grid<double>(c->B, c->sms, nt) : kh_tile_grid<float>(c->B, c->sms, nt);
         c->tlist = (int*)dev_alloc(c, 2 * (size_t)nt * sizeof(int), &err);
         if (!err) c->tctr = (unsigned*)dev_alloc(c, 4 * sizeof(unsigned), &err);
+        if (!err && kh_strips_ok(c->esz, cfg->nx, cfg->ny)) {
+            c->kh_full = (uint8_t*)work_alloc(c, (size_t)nt, &err);
+            if (!err) c->kh_hit = (uint8_t*)work_alloc(c, nb, &err);
+            if (!err) c->kh_cnt = (unsigned*)work_alloc(c, 3 * sizeof(unsigned), &err);
+        }
         if (err) {
             dba_destroy(c);
             return err;

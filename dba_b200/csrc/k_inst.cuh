@@ -215,11 +215,33 @@ int kh_tile_grid(int B, int sms, int ntiles)
     return B == 8 ? kh_tile_grid_b<R, 8>(sms, ntiles) : kh_tile_grid_b<R, 16>(sms, ntiles);
 }
 
+// full tiles by strips; DBA: the others by tiles
+template <int B>
+static cudaError_t kh_strips(bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P)
+{
+    const int sg = (g.nb + 255) / 256;
+    const KHPairK K = make_kh_pair(P.Kc);
+    const int H = KHStrip::rows(g.nx, g.ny);
+    const int units = ((g.nx + KHStrip::OUT - 1) / KHStrip::OUT) * ((g.ny + H - 1) / H);
+    const int ug = (units + KHStrip::NT / 32 - 1) / (KHStrip::NT / 32);
+    if (dba_mode) {
+        kh_strip_scan<B, true><<<sg, 256, 0, st>>>(g, f, P);
+        kh_strip_step<B, true><<<ug, KHStrip::NT, 0, st>>>(g, f, P, K, H);
+        kh_tile_step<float, B, true><<<grid, KHTile<float, B>::NT, KHTile<float, B>::smem, st>>>(g, f, P);
+    } else {
+        kh_strip_scan<B, false><<<sg, 256, 0, st>>>(g, f, P);
+        kh_strip_step<B, false><<<ug, KHStrip::NT, 0, st>>>(g, f, P, K, H);
+    }
+    return cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                            const KHTileP<R>& P)
 {
     if (!f.tlist || !f.tctr) return cudaErrorInvalidValue;
+    if constexpr (sizeof(R) == 4)
+        if (P.full) return B == 8 ? kh_strips<8>(dba_mode, grid, st, g, f, P) : kh_strips<16>(dba_mode, grid, st, g, f, P);
     // the scan lists the step's tiles (one thread per block), the tile kernel takes them
     const int sg = (int)(((long long)g.nb + 255) / 256 < 65535 ? ((long long)g.nb + 255) / 256 : 65535);
 #define XT(b)                                                                                          \

@@ -10,6 +10,7 @@
 #include "k_dendrite3.cuh"
 #include "k_dendrite_tile.cuh"
 #include "k_kh.cuh"
+#include "k_kh_strip.cuh"
 #include "k_kh_tile.cuh"
 #include "k_modelb.cuh"
 #include "k_modelb_fast.cuh"
@@ -74,6 +75,10 @@ inline bool kh_tiles_ok(int D, int B, int nx, int ny)
 {
     return D == 2 && (B == 8 || B == 16) && nx % 16 == 0 && ny % 16 == 0;
 }
+// Whether its fully active regions go through strips (k_kh_strip.cuh): FP32, and enough cells for
+// the strips' warps to fill the GPU.  us per step, DBA with every block active, tiles / strips:
+// 512^2 18.6 / 26, 1024^2 39.4 / 35.4, 2048^2 120 / 78.
+inline bool kh_strips_ok(int precision_bytes, int nx, int ny) { return precision_bytes == 4 && (long long)nx * ny >= 1 << 20; }
 template <typename R> int kh_tile_grid(int B, int sms, int ntiles);
 template <typename R>
 cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
