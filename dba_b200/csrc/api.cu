@@ -800,7 +800,7 @@ int dba_create(const dba_config* cfg, dba_ctx** out)
     }
     if (cfg->model == DBA_MODEL_MODELB && c->esz == 4 && cfg->tiles && modelb_tiles_ok(c->D, c->B, cfg->nx, cfg->ny)) {
         c->tiles = cfg->tiles == 2 ? 2 : 1;
-        c->grid = modelb_tile_grid(c->B, c->sms, (cfg->nx / 32) * (cfg->ny / 32));
+        c->grid = modelb_tile_grid(c->B, c->sms, ((cfg->nx + 31) / 32) * ((cfg->ny + 31) / 32));
     }
     if (cfg->model == DBA_MODEL_MODELB && c->esz == 4 && cfg->conserved && modelb_uses_fast<float>(c->D, c->B)) {
         c->lazy = true;

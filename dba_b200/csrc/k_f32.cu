@@ -19,7 +19,14 @@ cudaError_t launch_gather_lazy(cudaStream_t st, const GridP& g, int B, const flo
 
 bool modelb_tiles_ok(int D, int B, int nx, int ny)
 {
-    return D == 2 && (B == 8 || B == 16) && nx % MBTile<16>::T == 0 && ny % MBTile<16>::T == 0;
+    // Grids of whole tiles; or of whole blocks, two tiles across and 64 tiles in all: the last tiles
+    // then reach past the edge and continue with the first blocks, a single wrap away.  us per
+    // step, one block at a time / tiles: 1000 x 760 in 8^2 blocks, 44 % active 20.3 / 10.9, all
+    // 30.7 / 10.5; 400 x 272 in 16^2 blocks (117 tiles) 8.9 / 7.3; 200 x 136 in 8^2 blocks (35
+    // tiles) 6.2 / 6.6; 1920 x 1600 in 32^2 blocks 59.8 / 28.6.
+    if (D != 2 || (B != 8 && B != 16 && B != 32)) return false;
+    constexpr int T = MBTile<16>::T;
+    return (nx % T == 0 && ny % T == 0) || (nx >= 2 * T && ny >= 2 * T && (long long)nx * ny >= 64 * T * T);
 }
 
 template <int B>
@@ -70,7 +77,7 @@ cudaError_t launch_dendrite3_tiles(bool dba_mode, int grid, cudaStream_t st, con
 
 int modelb_tile_grid(int B, int sms, int ntiles)
 {
-    return B == 8 ? tile_grid_b<8>(sms, ntiles) : tile_grid_b<16>(sms, ntiles);
+    return B == 8 ? tile_grid_b<8>(sms, ntiles) : (B == 16 ? tile_grid_b<16>(sms, ntiles) : tile_grid_b<32>(sms, ntiles));
 }
 
 cudaError_t launch_modelb_tiles(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
@@ -90,7 +97,7 @@ cudaError_t launch_modelb_tiles(int B, bool dba_mode, int grid, cudaStream_t st,
         }                                                                                                         \
         return cudaGetLastError();                                                                                \
     }
-    XT(8) XT(16)
+    XT(8) XT(16) XT(32)
 #undef XT
     return cudaErrorInvalidValue;
 }

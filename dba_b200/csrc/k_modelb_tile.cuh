@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256 / R, 4)
 
     const int tid = threadIdx.x;
     const int G = gridDim.x;
-    const int ntx = g.nx / T, nty = g.ny / T, ntiles = ntx * nty;
+    const int ntx = (g.nx + T - 1) / T, nty = (g.ny + T - 1) / T, ntiles = ntx * nty;
     const size_t nx = (size_t)g.nx;
     const bool ghosts = g.ob0 > 0 || g.ob1 < g.nby;     // a slab with ghost block rows
     if (tid < 3) {
@@ -324,15 +324,16 @@ __global__ void __launch_bounds__(256 / R, 4)
         {
             const long long tl = blockIdx.x + (long long)G * (j0 + tid / NBT);
             const int kq = tid % NBT;
-            const bool valid = tl < ntiles;
             const int tile = (int)tl;
-            int act = 0, pp = 0, entry = 0;
+            const int stby = tile / ntx, stbx = tile - stby * ntx;
+            const int sbx = stbx * TB + kq % TB, by = stby * TB + kq / TB;
+            // the last tiles may reach past the grid: their blocks there are never listed
+            const bool valid = tl < ntiles && sbx < g.nbx && by < g.nby;
+            const int entry = stbx | (stby << 16);
+            int act = 0, pp = 0;
             if (valid) {
-                const int tby = tile / ntx, tbx = tile - tby * ntx;
-                const int b = (tbx * TB + kq % TB) + g.nbx * (tby * TB + kq / TB);
-                entry = tbx | (tby << 16);
+                const int b = sbx + g.nbx * by;
                 pp = f.par_cur[b];
-                const int by = tby * TB + kq / TB;
                 act = (by >= g.ob0 && by < g.ob1) ? (DBA ? (f.wake_cur[b] ? 1 : 0) : 1) : 0;
                 f.wake_clr[b] = 0;
                 if (!DBA) f.wake_nxt[b] = 1;
@@ -398,8 +399,10 @@ __global__ void __launch_bounds__(256 / R, 4)
             const float* sz = sy + SV;
             const bool own = (tm >> kb) & 1u;
             // potentials of this patch are recomputed where its block is active this step --
-            // listed here, or (a slab's ghost block, never listed) flagged by its owner
-            const bool fresh = own || (ghosts && s_nact[st][kb % TB + 1 + RB * (kb / TB + 1)]);
+            // listed here, or (a slab's ghost block, never listed) flagged by its owner, or (past
+            // the grid's edge, where the tile continues with the first blocks) listed in its own tile
+            const bool past = X0 + T > g.nx || Y0 + T > g.ny;
+            const bool fresh = own || ((ghosts || past) && s_nact[st][kb % TB + 1 + RB * (kb / TB + 1)]);
 
             // ---- potentials of this patch (Calc_mu, kernel.cu:371-388)
             // Laplacians of the patch: every lane of the warp takes part (the row
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(256 / R, 4)
                 // inactive block inside the tile: its persisted ring (stale potentials)
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const size_t gi = (size_t)(X0 + lx0) + nx * (size_t)(Y0 + ly0 + r);
+                    const size_t gi = (size_t)wrap_p(X0 + lx0, g.nx) + nx * (size_t)wrap_p(Y0 + ly0 + r, g.ny);
                     const int mi = (ly0 + r + 1) * MP + lx0 + 4;
 #pragma unroll
                     for (int q = 0; q < 3; ++q)
