@@ -27,7 +27,7 @@ UNITS = [
     ("noalloc.cu", ["-fmad=false"]),
     ("batch.cu", ["-fmad=false"]),
 ]
-HEADERS = ["fpmath.h", "fpmath_coeffs.h", "k_common.cuh", "k_dendrite.cuh", "k_dendrite3.cuh", "k_modelb.cuh", "k_kh.cuh",
+HEADERS = ["fpmath.h", "fpmath_coeffs.h", "k_common.cuh", "k_dendrite.cuh", "k_dendrite2.cuh", "k_dendrite3.cuh", "k_modelb.cuh", "k_kh.cuh",
            "k_reduce.cuh", "k_inst.cuh", "launch.h", "k_modelb_fast.cuh", "k_modelb_tile.cuh", "k_kh_tile.cuh", "k_kh_strip.cuh", "k_dendrite_tile.cuh", "k_batch.cuh", "k_post.cuh", "k_pair.cuh"]
 
 

@@ -67,7 +67,7 @@ struct dba_ctx {
     float* fstaging = nullptr;        // dba_read_field_f32: a field as floats (allocated on first use)
     bool kh_tiles = false;            // KH one-kernel step on 16x16-cell tiles (k_kh_tile.cuh)
     bool den_tiles = false;           // FP32 3-D dendrite on 32x8x8-cell tiles (k_dendrite_tile.cuh)
-    bool den3_list = false;           // 3-D dendrite through the general tile kernel: list in tlist, counts in tctr[step % 2]
+    bool den3_list = false;           // dendrite through the general tile kernels: list in tlist, counts in tctr[step % 2]
     double lazy_ncells = 0;           // divisor of the FP32 conserved offset when the context is a slab of a
                                       //   larger domain (dba_slab_rows); 0: this context's cells
     int* tlist = nullptr;             // tile queue of the tile kernels that take tiles dynamically
@@ -328,7 +328,7 @@ cudaError_t enqueue_step_t(dba_ctx* c, long s, bool dba_mode)
     case DBA_MODEL_DENDRITE:
         if constexpr (sizeof(R) == 4)
             if (c->den_tiles) return launch_dendrite3_tiles(dba_mode, c->grid, c->st, c->g, f, den_params<float>(c));
-        return launch_dendrite<R>(c->D, c->B, dba_mode, c->grid, c->st, c->g, f, den_params<R>(c));
+        return launch_dendrite<R>(c->D, c->B, dba_mode, c->grid, c->sms, c->st, c->g, f, den_params<R>(c));
     case DBA_MODEL_MODELB: {
         MBP<R> P = mb_params<R>(c, dba_mode);
         LazyP L = lazy_params(c, s, P.conserved != 0);
@@ -775,7 +775,7 @@ int dba_create(const dba_config* cfg, dba_ctx** out)
             c->grid = dendrite3_tile_grid(c->sms, nt);
         } else if (listed) {
             c->den3_list = true;
-            c->tlist = (int*)work_alloc(c, (size_t)nt * kDen3Entry * sizeof(int), &err);
+            c->tlist = (int*)work_alloc(c, (size_t)nt * kDenEntry * sizeof(int), &err);
             if (!err) c->tctr = (unsigned*)work_alloc(c, 4 * sizeof(unsigned), &err);
         }
         if (err) {
@@ -1351,7 +1351,7 @@ int dba_step_profiled(dba_ctx* c, int nsteps, int mode, dba_prof* out)
         cudaError_t r = cudaEventRecord(e[0], c->st);
         if (r == cudaSuccess) {
             if (c->esz == 8) {
-                if (c->cfg.model == DBA_MODEL_DENDRITE) r = launch_dendrite<double>(c->D, c->B, dba_mode, c->grid, c->st, c->g, f, den_params<double>(c));
+                if (c->cfg.model == DBA_MODEL_DENDRITE) r = launch_dendrite<double>(c->D, c->B, dba_mode, c->grid, c->sms, c->st, c->g, f, den_params<double>(c));
                 else if (c->cfg.model == DBA_MODEL_MODELB) {
                     MBP<double> P = mb_params<double>(c, dba_mode);
                     LazyP L = lazy_params(c, s, P.conserved != 0);
@@ -1365,7 +1365,7 @@ int dba_step_profiled(dba_ctx* c, int nsteps, int mode, dba_prof* out)
             } else {
                 if (c->cfg.model == DBA_MODEL_DENDRITE)
                     r = c->den_tiles ? launch_dendrite3_tiles(dba_mode, c->grid, c->st, c->g, f, den_params<float>(c))
-                                     : launch_dendrite<float>(c->D, c->B, dba_mode, c->grid, c->st, c->g, f, den_params<float>(c));
+                                     : launch_dendrite<float>(c->D, c->B, dba_mode, c->grid, c->sms, c->st, c->g, f, den_params<float>(c));
                 else if (c->cfg.model == DBA_MODEL_MODELB) {
                     MBP<float> P = mb_params<float>(c, dba_mode);
                     LazyP L = lazy_params(c, s, P.conserved != 0);

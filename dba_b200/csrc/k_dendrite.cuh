@@ -1,5 +1,5 @@
-// k_dendrite.cuh -- one fused step of the Kobayashi p/T dendrite model over
-// the active blocks (reference: example_Dendritic_growth/kernel.cu).
+// k_dendrite.cuh -- point formulas of the Kobayashi p/T dendrite model
+// (reference: example_Dendritic_growth/kernel.cu), shared by its step kernels.
 //
 // The reference runs four kernels and a host sync per DBA step:
 //   Evolve_p_wakeup (:322)  p_new for p-active blocks
@@ -8,12 +8,12 @@
 //   Wakeup_Next (:496)      commit p/T of active blocks, per-block tests
 //                           metric_p <= p_new <= 1-metric_p and |T_new-T| >= metric_T
 //   Wakeup_Neighbor (:577)  wake self + 6 face neighbours for the next step
-// Here one kernel does all of it: each active block and its 1-cell halo are
-// staged in shared memory, p and T are advanced (Jacobi: every read sees the
-// start-of-step values, which live in each block's current ping-pong buffer),
-// results go to the block's other buffer (no commit copy), the wake-up tests
-// are block-wide ORs in shared memory and the neighbour wake-up is a scatter
-// into next step's flag array.  A p-active block that is not T-active keeps
+// The step kernels (k_dendrite2.cuh, k_dendrite3.cuh, k_dendrite_tile.cuh, k_batch.cuh) do all of
+// it in one: active blocks and a 1-cell halo are staged in shared memory, p and T are
+// advanced (Jacobi: every read sees the start-of-step values, which live in each block's
+// current ping-pong buffer), results go to the block's other buffer (no commit copy), the
+// wake-up tests are ORs over a block in shared memory and the neighbour wake-up is a
+// scatter into next step's flag array.  A p-active block that is not T-active keeps
 // its T untouched, exactly as the reference, whose T_new is not committed then.
 // Regular mode (DBA=false) uses the reference's mode-0 rounding order for T
 // (T + dt lapT + p_new - p, kernel.cu:289).
@@ -163,155 +163,6 @@ __device__ __forceinline__ R den_T_new(R Tc, R Txp, R Txm, R Typ, R Tym, R Tzp, 
         return p_active ? da(Tn, ds(pn, pc)) : Tn;
     }
     return ds(da(da(Tc, dm(dt, lapT)), pn), pc);
-}
-
-template <typename R, int D, int B, bool DBA>
-__global__ void __launch_bounds__(kThreads) dendrite_step(GridP g, FlagP f, DenP<R> P)
-{
-    constexpr int NT = kThreads;
-    constexpr int V = ipow(B, D);
-    constexpr int E = B + 2;
-    constexpr int TV = ipow(E, D);
-    constexpr int K = V >= NT ? 1 : NT / V;
-    constexpr int CPT = V >= NT ? V / NT : 1;
-    constexpr int SY = E, SZ = (D == 3) ? E * E : 0;
-
-    __shared__ R sp[K * TV];
-    __shared__ R sT[K * TV];
-    __shared__ int s_list[NT], s_lmeta[NT];
-    __shared__ int s_cnt;
-    __shared__ int s_blk[K], s_meta[K], s_np[K], s_nT[K];
-    __shared__ int s_bx[K], s_by[K], s_bz[K];   // block coordinates of the round's blocks
-    static_assert(K * 14 <= NT, "one wake-up scatter thread per block, channel and neighbour");
-
-    const int tid = threadIdx.x;
-    const int G = gridDim.x;
-    const int nb = g.nb;
-    const R f0 = (R)P.f0, f1 = (R)P.f1, f2 = (R)P.f2, f3 = (R)P.f3;
-    const R dt = (R)P.dt, delta = (R)P.delta, eps2 = (R)P.eps2, gam = (R)P.gamma;
-    const R thr_p = (R)P.thr_p, thr_p_hi = (R)P.thr_p_hi, thr_T = (R)P.thr_T;
-
-    for (long long j0 = 0; blockIdx.x + (long long)G * j0 < nb; j0 += NT) {
-        const long long bl = blockIdx.x + (long long)G * (j0 + tid);
-        const bool valid = bl < nb;
-        const int b = (int)bl;
-        int act = 0, meta = 0;
-        if (valid) {
-            int pp = f.par_cur[b], pT = f.par_cur[nb + b];
-            act = DBA ? ((f.wake_cur[b] ? 1 : 0) | (f.wake_cur[nb + b] ? 2 : 0)) : 3;
-            f.wake_clr[b] = 0;
-            f.wake_clr[nb + b] = 0;
-            if (!DBA) {
-                f.wake_nxt[b] = 1;
-                f.wake_nxt[nb + b] = 1;
-            }
-            f.par_nxt[b] = (uint8_t)(pp ^ (act & 1));
-            f.par_nxt[nb + b] = (uint8_t)(pT ^ ((act >> 1) & 1));
-            meta = act | (pp << 2) | (pT << 3);
-        }
-        count_stats(f.stats, act, valid);
-        if (tid == 0) s_cnt = 0;
-        __syncthreads();
-        list_append(valid && act, b, meta, s_list, s_lmeta, &s_cnt);
-        __syncthreads();
-        const int cnt = s_cnt;
-
-        for (int q0 = 0; q0 < cnt; q0 += K) {
-            if (tid < K) {
-                int q = q0 + tid;
-                const int blk = q < cnt ? s_list[q] : -1;
-                s_blk[tid] = blk;
-                s_meta[tid] = q < cnt ? s_lmeta[q] : 0;
-                if (blk >= 0) {
-                    s_bx[tid] = blk % g.nbx;
-                    s_by[tid] = (blk / g.nbx) % g.nby;
-                    s_bz[tid] = blk / (g.nbx * g.nby);
-                }
-                s_np[tid] = 0;
-                s_nT[tid] = 0;
-            }
-            __syncthreads();
-            // stage p and T of each block plus a 1-cell halo (owner's current buffer).  2-D
-            // grids (small, L2-resident at the workloads' sizes) load both buffers beside the
-            // owner's parity and select afterwards, so the staging waits for one memory
-            // round trip instead of two; 3-D grids load the parity first
-            for (int i = tid; i < K * TV; i += NT) {
-                const int k = i / TV;
-                if (s_blk[k] < 0) continue;
-                const int j = i - k * TV;
-                const int lx = j % E, ly = (j / E) % E, lz = (D == 3) ? j / (E * E) : 0;
-                const int gx = wrapc(s_bx[k] * B + lx - 1, g.nx, g.bc);
-                const int gy = wrapc(s_by[k] * B + ly - 1, g.ny, g.bc);
-                const int gz = (D == 3) ? wrapc(s_bz[k] * B + lz - 1, g.nz, g.bc) : 0;
-                const int ob = gx / B + g.nbx * (gy / B + g.nby * ((D == 3) ? gz / B : 0));
-                const size_t gi = (size_t)gx + (size_t)g.nx * ((size_t)gy + (size_t)g.ny * gz);
-                if constexpr (D == 2) {
-                    const uint8_t pp = f.par_cur[ob], pT = f.par_cur[nb + ob];
-                    const R p0 = P.p[0][gi], p1 = P.p[1][gi], T0 = P.T[0][gi], T1 = P.T[1][gi];
-                    sp[i] = pp ? p1 : p0;
-                    sT[i] = pT ? T1 : T0;
-                } else {
-                    sp[i] = (f.par_cur[ob] ? P.p[1] : P.p[0])[gi];
-                    sT[i] = (f.par_cur[nb + ob] ? P.T[1] : P.T[0])[gi];
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int c = 0; c < CPT; ++c) {
-                const int k = (V >= NT) ? 0 : tid / V;
-                const int v = (V >= NT) ? tid + c * NT : tid - k * V;
-                const int blk = s_blk[k];
-                if (blk < 0) continue;
-                const int m = s_meta[k];
-                const int lx = v % B, ly = (v / B) % B, lz = (D == 3) ? v / (B * B) : 0;
-                const int ti = k * TV + (lx + 1) + SY * (ly + 1) + SZ * (lz + 1);
-                const int bx = s_bx[k], by = s_by[k], bz = s_bz[k];
-                const size_t gi = (size_t)(bx * B + lx) +
-                                  (size_t)g.nx * ((size_t)(by * B + ly) + (size_t)g.ny * (size_t)((D == 3) ? bz * B + lz : 0));
-                const R pc = sp[ti], Tc = sT[ti];
-                R pn = pc;
-                if (m & 1) {   // Evolve_p (kernel.cu:220-241)
-                    if constexpr (std::is_same<R, float>::value)
-                        pn = den_p_f32<D>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + SY], sp[ti - SY], sp[ti + SZ],
-                                          sp[ti - SZ], P.c32);
-                    else
-                        pn = den_p_new<R>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + SY], sp[ti - SY], sp[ti + SZ],
-                                          sp[ti - SZ], f0, f1, f2, f3, dt, delta, eps2, gam);
-                    ((m & 4) ? P.p[0] : P.p[1])[gi] = pn;
-                    if (pn >= thr_p && pn <= thr_p_hi) s_np[k] = 1;
-                    if (!isfinite(pn)) raise_status(f.status, 5);
-                }
-                if (m & 2) {   // Evolve_T (kernel.cu:286-289, :468-489)
-                    R Tn;
-                    if constexpr (std::is_same<R, float>::value)
-                        Tn = den_T_f32<D, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + SY], sT[ti - SY], sT[ti + SZ],
-                                               sT[ti - SZ], (m & 1) != 0, pn, pc, P.c32);
-                    else
-                        Tn = den_T_new<R, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + SY], sT[ti - SY], sT[ti + SZ],
-                                               sT[ti - SZ], (m & 1) != 0, pn, pc, f1, dt);
-                    ((m & 8) ? P.T[0] : P.T[1])[gi] = Tn;
-                    if (fabs(Tn - Tc) >= thr_T) s_nT[k] = 1;
-                    if (!isfinite(Tn)) raise_status(f.status, 5);
-                }
-            }
-            __syncthreads();
-            // wake-up tests and scatter: self + 6 faces per channel (kernel.cu:577-634), one
-            // neighbour per thread (thread (2 k + ch) * 7 + n), from the block coordinates
-            if (DBA && tid < K * 14) {
-                const int k = tid / 14, r = tid - k * 14, ch = r / 7, n = r - ch * 7;
-                const int blk = s_blk[k];
-                if (blk >= 0 && ((s_meta[k] >> ch) & 1)) {
-                    const int t = ch ? s_nT[k] : s_np[k];
-                    if (n == 0) f.next[(size_t)ch * nb + blk] = (uint8_t)t;
-                    if (t) {
-                        const int nbk = block_nb_k(g, s_bx[k], s_by[k], s_bz[k], n);
-                        if (nbk >= 0) f.wake_nxt[(size_t)ch * nb + nbk] = 1;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
 }
 
 }  // namespace dba

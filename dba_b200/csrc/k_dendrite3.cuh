@@ -29,7 +29,7 @@
 
 namespace dba {
 
-constexpr int kDen3Entry = 8;                            // ints per entry of the tile list
+constexpr int kDenEntry = 8;                             // ints per entry of the tile list
 
 template <typename R, int B>
 struct Den3 {
@@ -49,7 +49,6 @@ struct Den3 {
     static constexpr int IPB = V / (32 * NZ);
     static constexpr int NPR = TX / PC + 2;              // pieces per staged row: x from -PC to TX + PC - 1
     static constexpr int PP = NPR * SH, ZP = NT / PP;    // pieces of a plane, planes staged at once
-    static constexpr int LE = kDen3Entry;                     // ints per list entry
     static constexpr size_t smem = sizeof(R) * 2 * SV;
     static constexpr int MINB = sizeof(R) == 8 ? 3 : 5;  // resident CTAs per SM
     static_assert(ZP >= 1 && NBT <= 32 && (NBT & (NBT - 1)) == 0 && TX % B == 0 && 8 % B == 0 && B % PC == 0 && 4 % PC == 0, "tile shape");
@@ -59,10 +58,9 @@ struct Den3 {
 // warp (all its lanes call): parity flip of active blocks, clearing of the flag array two
 // steps ahead, activity counts.  Returns the tile's masks: blocks active in p, in T,
 // parity in p, in T.  (x, y, z) the tile, k the thread's block in it; in: the tile exists.
-template <typename R, int B, bool DBA>
-__device__ __forceinline__ uint4 den3_blocks(const GridP& g, const FlagP& f, bool in, int tx, int ty, int tz, int k)
+template <typename S, bool DBA>
+__device__ __forceinline__ uint4 den_blocks(const GridP& g, const FlagP& f, bool in, int tx, int ty, int tz, int k)
 {
-    using S = Den3<R, B>;
     constexpr int NBT = S::NBT;
     const int nb = g.nb;
     const int x = tx * S::NBX + k % S::NBX, y = ty * S::NBY + (k / S::NBX) % S::NBY, z = tz * S::NBZ + k / (S::NBX * S::NBY);
@@ -95,16 +93,15 @@ __device__ __forceinline__ uint4 den3_blocks(const GridP& g, const FlagP& f, boo
 
 // Scan of one step: the bookkeeping, and one list entry per tile with an active block: [0]
 // its x, [1..4] its masks, [5] [6] its y and z (in tiles).
-template <typename R, int B, bool DBA>
-__global__ void __launch_bounds__(256) dendrite3_scan(GridP g, FlagP f, int ntiles)
+template <typename S, bool DBA>
+__global__ void __launch_bounds__(256) dendrite_scan(GridP g, FlagP f, int ntiles)
 {
-    using S = Den3<R, B>;
     const int lane = threadIdx.x & 31;
     const int ntx = (g.nx + S::TX - 1) / S::TX, nty = (g.ny + S::TY - 1) / S::TY;
     const int it = blockIdx.x * 256 + threadIdx.x;       // the grid covers ntiles * NBT items
     const int tile = it / S::NBT, k = it % S::NBT;
     const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
-    const uint4 m = den3_blocks<R, B, DBA>(g, f, tile < ntiles, tx, ty, tz, k);
+    const uint4 m = den_blocks<S, DBA>(g, f, tile < ntiles, tx, ty, tz, k);
     const bool take = k == 0 && (m.x | m.y) != 0;
     const unsigned mt = __ballot_sync(0xffffffffu, take);
     if (mt == 0) return;
@@ -114,7 +111,7 @@ __global__ void __launch_bounds__(256) dendrite3_scan(GridP g, FlagP f, int ntil
     if (take) {
         const unsigned e = base + (unsigned)__popc(mt & ((1u << lane) - 1u));
         if (e < (unsigned)ntiles) {
-            int* d = f.tlist + (size_t)e * S::LE;
+            int* d = f.tlist + (size_t)e * kDenEntry;
             *reinterpret_cast<int4*>(d) = make_int4(tx, (int)m.x, (int)m.y, (int)m.z);
             *reinterpret_cast<int4*>(d + 4) = make_int4((int)m.w, ty, tz, 0);
         }
@@ -213,13 +210,13 @@ __global__ void __launch_bounds__(256, Den3<R, B>::MINB) dendrite3_step(GridP g,
     for (int i = blockIdx.x, it = 0; i < cnt; i += gridDim.x, it ^= 1) {
         int4 ea, eb;
         if (LIST) {
-            ea = __ldcg(reinterpret_cast<const int4*>(f.tlist + (size_t)i * S::LE));
-            eb = __ldcg(reinterpret_cast<const int4*>(f.tlist + (size_t)i * S::LE + 4));
+            ea = __ldcg(reinterpret_cast<const int4*>(f.tlist + (size_t)i * kDenEntry));
+            eb = __ldcg(reinterpret_cast<const int4*>(f.tlist + (size_t)i * kDenEntry + 4));
         } else {
             const int ntx = (g.nx + S::TX - 1) / S::TX, nty = (g.ny + S::TY - 1) / S::TY;
             ea.x = i % ntx; eb.y = (i / ntx) % nty; eb.z = i / (ntx * nty);
             if (tid < 32) {
-                const uint4 m = den3_blocks<R, B, DBA>(g, f, tid < S::NBT, ea.x, eb.y, eb.z, tid);
+                const uint4 m = den_blocks<S, DBA>(g, f, tid < S::NBT, ea.x, eb.y, eb.z, tid);
                 if (tid == 0) s_mask = m;
             }
             __syncthreads();

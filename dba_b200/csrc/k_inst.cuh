@@ -73,12 +73,22 @@ static cudaError_t den3_launch(bool dba_mode, int grid, cudaStream_t st, const G
     const int ng = 8 * grid < nt ? 8 * grid : nt;
     const int sg = (int)(((long long)nt * S::NBT + 255) / 256);
     if (dba_mode) {
-        dendrite3_scan<R, B, true><<<sg, 256, 0, st>>>(g, f, nt);
+        dendrite_scan<S, true><<<sg, 256, 0, st>>>(g, f, nt);
         dendrite3_step<R, B, true, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
     } else {
-        dendrite3_scan<R, B, false><<<sg, 256, 0, st>>>(g, f, nt);
+        dendrite_scan<S, false><<<sg, 256, 0, st>>>(g, f, nt);
         dendrite3_step<R, B, false, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
     }
+    return cudaGetLastError();
+}
+
+template <typename R, int B>
+static cudaError_t den2_launch(bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f, const DenP<R>& P)
+{
+    const int nt = dendrite2_tiles(B, g.nx, g.ny);
+    if (!dendrite2_tiled(sizeof(R), dba_mode, nt, sms)) dendrite2_owned<R, B><<<grid, kThreads, 0, st>>>(g, f, P);
+    else if (dba_mode) dendrite2_step<R, B, true><<<nt, kThreads, 0, st>>>(g, f, P);
+    else dendrite2_step<R, B, false><<<nt, kThreads, 0, st>>>(g, f, P);
     return cudaGetLastError();
 }
 
@@ -87,7 +97,7 @@ int step_grid(int model, int D, int B, int sms)
 {
 #define XD(d, b) if (D == d && B == b) { \
     if constexpr (d == 3) return den3_prepare<R, b>(sms); \
-    else return grid_of<R>((const void*)dendrite_step<R, d, b, true>, 0, sms); }
+    else return grid_of<R>((const void*)dendrite2_owned<R, b>, 0, sms); }
 #define XM(d, b) if (D == d && B == b) { \
     if constexpr (sizeof(R) == 4 && d == 2) return grid_of<R>((const void*)modelb_fast_step<b, true>, MBFastShape<b>::smem, sms); \
     else return mb_prepare<R, d, b>(sms); }
@@ -102,17 +112,13 @@ int step_grid(int model, int D, int B, int sms)
 }
 
 template <typename R>
-cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
+cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f,
                             const DenP<R>& P)
 {
 #define XD(d, b)                                                                   \
     if (D == d && B == b) {                                                        \
         if constexpr (d == 3) return den3_launch<R, b>(dba_mode, grid, st, g, f, P); \
-        else {                                                                     \
-            if (dba_mode) dendrite_step<R, d, b, true><<<grid, kThreads, 0, st>>>(g, f, P); \
-            else dendrite_step<R, d, b, false><<<grid, kThreads, 0, st>>>(g, f, P); \
-        }                                                                          \
-        return cudaGetLastError();                                                 \
+        else return den2_launch<R, b>(dba_mode, grid, sms, st, g, f, P);           \
     }
     DBA_DEN_SHAPES(XD)
 #undef XD
@@ -439,7 +445,7 @@ template cudaError_t launch_batch_step<REAL_T>(int, int, int, cudaStream_t, cons
 template cudaError_t launch_batch_tips<REAL_T>(cudaStream_t, const BatchP&, const uint8_t*, int, double*);
 template bool shape_supported<REAL_T>(int, int, int);
 template int step_grid<REAL_T>(int, int, int, int);
-template cudaError_t launch_dendrite<REAL_T>(int, int, bool, int, cudaStream_t, const GridP&, const FlagP&, const DenP<REAL_T>&);
+template cudaError_t launch_dendrite<REAL_T>(int, int, bool, int, int, cudaStream_t, const GridP&, const FlagP&, const DenP<REAL_T>&);
 template cudaError_t launch_modelb<REAL_T>(int, int, bool, int, cudaStream_t, const GridP&, const FlagP&, const MBP<REAL_T>&, const LazyP*, int);
 template bool modelb_uses_fast<REAL_T>(int, int);
 template cudaError_t launch_kh<REAL_T>(int, bool, int, cudaStream_t, const GridP&, const FlagP&, const KHP<REAL_T>&);

@@ -7,6 +7,7 @@
 
 #include "k_common.cuh"
 #include "k_dendrite.cuh"
+#include "k_dendrite2.cuh"
 #include "k_dendrite3.cuh"
 #include "k_dendrite_tile.cuh"
 #include "k_kh.cuh"
@@ -26,7 +27,7 @@ enum { MODEL_DENDRITE = 0, MODEL_MODELB = 1, MODEL_KH = 2 };
 template <typename R> bool shape_supported(int model, int D, int B);
 template <typename R> int step_grid(int model, int D, int B, int sms);
 template <typename R>
-cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
+cudaError_t launch_dendrite(int D, int B, bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f,
                             const DenP<R>& P);
 // FP32 3-D dendrite on double-buffered 32x8x8-cell tiles (k_dendrite_tile.cuh), for grids that
 // need a tile list (dendrite3_listed)
@@ -46,6 +47,13 @@ inline int dendrite3_tiles(int nx, int ny, int nz) { return ((nx + 31) / 32) * (
 // FP32 8^3 grids that need a list take the double-buffered tiles of k_dendrite_tile.cuh instead:
 // 512^3 dense 745 against 779 us, 256^3 106 against 107, but 200x136x104 29.6 against 25.1.
 inline bool dendrite3_listed(int tiles, int resident) { return tiles > 4 * resident; }
+// 2-D: whether a step goes by tiles (k_dendrite2.cuh, with the figures): every regular step; DBA steps
+// while the tiles are about as many as the GPU holds at once (148 x 5 in FP64, 148 x 6 in FP32)
+inline int dendrite2_tiles(int B, int nx, int ny) { return ((nx + 31) / 32) * (B > 8 ? ny / B : (ny + 7) / 8); }
+inline bool dendrite2_tiled(int precision_bytes, bool dba_mode, int tiles, int sms)
+{
+    return !dba_mode || tiles <= (precision_bytes == 8 ? 5 * sms : 9 * sms);
+}
 cudaError_t launch_dendrite3_tiles(bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                                    const DenP<float>& P);
 // FP32 2-D uses the fast kernels (lazy conserved correction, reduction fused):

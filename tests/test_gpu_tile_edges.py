@@ -1,4 +1,4 @@
-"""The 3-D dendrite tile kernel and the two Model B kernels where their tiles end: grids that
+"""The dendrite tile kernels and the two Model B kernels where their tiles end: grids that
 are multiples of the block edge only, one tile or several, the smallest grids, partial
 activity.  FP64 must equal the CPU restatement bit for bit, flags at every step; FP32 stays
 within the tolerances of test_gpu_parity.py (2e-5 for the dendrite's fields, relative L2 1e-4
@@ -26,8 +26,11 @@ def _seed(nx, ny, nz, r):
     (36, 20, 12, 4, 1, 0, 0), (36, 20, 12, 4, 1, 1, 0), (40, 24, 16, 8, 1, 0, 0), (72, 24, 8, 8, 1, 1, 0),
     (4, 4, 4, 4, 1, 0, 0), (8, 8, 8, 8, 1, 1, 0), (68, 12, 20, 4, 0, 1, 0), (40, 16, 24, 8, 0, 0, 0),
     (36, 20, 12, 4, 1, 1, 1), (68, 12, 20, 4, 0, 0, 1), (40, 24, 16, 8, 1, 1, 1), (200, 128, 144, 4, 1, 0, 0),
-    (136, 144, 168, 8, 1, 1, 0)])                       # the last two work from a tile list
-def test_dendrite3_tile_edges(nx, ny, nz, B, mode, bc, precision):
+    (136, 144, 168, 8, 1, 1, 0),                         # the last two work from a tile list
+    (36, 20, 1, 4, 1, 1, 0), (36, 20, 1, 4, 0, 0, 0), (40, 24, 1, 8, 1, 0, 0), (48, 80, 1, 16, 1, 1, 0),
+    (96, 32, 1, 32, 1, 0, 0), (4, 4, 1, 4, 1, 1, 0), (40, 24, 1, 8, 1, 1, 1), (48, 80, 1, 16, 0, 1, 1),
+    (1000, 256, 1, 8, 1, 1, 0), (1000, 260, 1, 4, 1, 0, 0)])   # these two have more tiles than a DBA step takes by tile
+def test_dendrite_tile_edges(nx, ny, nz, B, mode, bc, precision):
     p, T = _seed(nx, ny, nz, 3.0 if nx < 100 else 12.0)
     o = OracleDendrite(nx, ny, nz, B, DEN, bc=bc)
     o.set_fields(p, T)
