@@ -33,12 +33,19 @@ template <int B>
 static int tile_grid_b(int sms, int ntiles)
 {
     const size_t sm = MBTile<B>::smem;
-    cudaFuncSetAttribute(modelb_tile_step<B, kMBTileRows, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(modelb_tile_step<B, kMBTileRows, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(modelb_tile_step<B, kMBTileRows, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(modelb_tile_step<B, kMBTileRows, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    auto allow = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); };
+    allow(modelb_tile_step<B, kMBTileRows, true, false, false>);
+    allow(modelb_tile_step<B, kMBTileRows, false, false, false>);
+    allow(modelb_tile_step<B, kMBTileRows, true, true, false>);
+    allow(modelb_tile_step<B, kMBTileRows, false, true, false>);
+    if constexpr (B < 32) {
+        allow(modelb_tile_step<B, kMBTileRows, true, false, true>);
+        allow(modelb_tile_step<B, kMBTileRows, false, false, true>);
+        allow(modelb_tile_step<B, kMBTileRows, true, true, true>);
+        allow(modelb_tile_step<B, kMBTileRows, false, true, true>);
+    }
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, modelb_tile_step<B, kMBTileRows, true, false>, MBTile<B>::NT,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, modelb_tile_step<B, kMBTileRows, true, false, false>, MBTile<B>::NT,
                                                       sm) != cudaSuccess ||
         occ < 1)
         occ = 1;
@@ -80,25 +87,34 @@ int modelb_tile_grid(int B, int sms, int ntiles)
     return B == 8 ? tile_grid_b<8>(sms, ntiles) : (B == 16 ? tile_grid_b<16>(sms, ntiles) : tile_grid_b<32>(sms, ntiles));
 }
 
+template <int B, bool RAG>
+static cudaError_t modelb_tiles(bool dba_mode, bool bulk, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
+                                const MBFastP& P, const MBFastBuf& Q, const LazyP& L)
+{
+    const MBPairP K = make_pair_params(P);
+    const size_t sm = MBTile<B>::smem;
+    const int nt = MBTile<B>::NT;
+    if (bulk) {
+        if (dba_mode) modelb_tile_step<B, kMBTileRows, true, true, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
+        else modelb_tile_step<B, kMBTileRows, false, true, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
+    } else {
+        if (dba_mode) modelb_tile_step<B, kMBTileRows, true, false, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
+        else modelb_tile_step<B, kMBTileRows, false, false, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
+    }
+    return cudaGetLastError();
+}
+
 cudaError_t launch_modelb_tiles(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                                 const MBFastP& P, const MBFastBuf& Q, const LazyP& L, bool bulk)
 {
-    const MBPairP K = make_pair_params(P);
-#define XT(b)                                                                                                     \
-    if (B == b) {                                                                                                 \
-        const size_t sm = MBTile<b>::smem;                                                                        \
-        const int nt = MBTile<b>::NT;                                                                             \
-        if (bulk) {                                                                                               \
-            if (dba_mode) modelb_tile_step<b, kMBTileRows, true, true><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);   \
-            else modelb_tile_step<b, kMBTileRows, false, true><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);           \
-        } else {                                                                                                  \
-            if (dba_mode) modelb_tile_step<b, kMBTileRows, true, false><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);  \
-            else modelb_tile_step<b, kMBTileRows, false, false><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);          \
-        }                                                                                                         \
-        return cudaGetLastError();                                                                                \
-    }
-    XT(8) XT(16) XT(32)
-#undef XT
+    const bool rag = g.nx % 32 != 0 || g.ny % 32 != 0;
+    if (B == 8)
+        return rag ? modelb_tiles<8, true>(dba_mode, bulk, grid, st, g, f, P, Q, L)
+                   : modelb_tiles<8, false>(dba_mode, bulk, grid, st, g, f, P, Q, L);
+    if (B == 16)
+        return rag ? modelb_tiles<16, true>(dba_mode, bulk, grid, st, g, f, P, Q, L)
+                   : modelb_tiles<16, false>(dba_mode, bulk, grid, st, g, f, P, Q, L);
+    if (B == 32) return modelb_tiles<32, false>(dba_mode, bulk, grid, st, g, f, P, Q, L);
     return cudaErrorInvalidValue;
 }
 

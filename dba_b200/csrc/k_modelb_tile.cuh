@@ -193,7 +193,8 @@ __device__ __forceinline__ void mbar_wait(unsigned long long* m, unsigned parity
 // BULK: stage each tile row as one bulk copy per block segment (cp.async.bulk, completion
 // on a per-stage mbarrier), issued by one thread per staged row and field; otherwise
 // 16-byte cp.async pieces spread over the CTA
-template <int B, int R, bool DBA, bool BULK>
+// RAG: the last tiles may reach past the grid (its edges are multiples of B, not of T)
+template <int B, int R, bool DBA, bool BULK, bool RAG>
 __global__ void __launch_bounds__(256 / R, 4)
     modelb_tile_step(GridP g, FlagP f, MBFastP P, MBPairP K, MBFastBuf Q, LazyP L)
 {
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(256 / R, 4)
             const int stby = tile / ntx, stbx = tile - stby * ntx;
             const int sbx = stbx * TB + kq % TB, by = stby * TB + kq / TB;
             // the last tiles may reach past the grid: their blocks there are never listed
-            const bool valid = tl < ntiles && sbx < g.nbx && by < g.nby;
+            const bool valid = tl < ntiles && (!RAG || (sbx < g.nbx && by < g.nby));
             const int entry = stbx | (stby << 16);
             int act = 0, pp = 0;
             if (valid) {
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(256 / R, 4)
             // potentials of this patch are recomputed where its block is active this step --
             // listed here, or (a slab's ghost block, never listed) flagged by its owner, or (past
             // the grid's edge, where the tile continues with the first blocks) listed in its own tile
-            const bool past = X0 + T > g.nx || Y0 + T > g.ny;
+            const bool past = RAG && (X0 + T > g.nx || Y0 + T > g.ny);
             const bool fresh = own || ((ghosts || past) && s_nact[st][kb % TB + 1 + RB * (kb / TB + 1)]);
 
             // ---- potentials of this patch (Calc_mu, kernel.cu:371-388)
@@ -434,7 +435,8 @@ __global__ void __launch_bounds__(256 / R, 4)
                 // inactive block inside the tile: its persisted ring (stale potentials)
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const size_t gi = (size_t)wrap_p(X0 + lx0, g.nx) + nx * (size_t)wrap_p(Y0 + ly0 + r, g.ny);
+                    const size_t gi = RAG ? (size_t)wrap_p(X0 + lx0, g.nx) + nx * (size_t)wrap_p(Y0 + ly0 + r, g.ny)
+                                          : (size_t)(X0 + lx0) + nx * (size_t)(Y0 + ly0 + r);
                     const int mi = (ly0 + r + 1) * MP + lx0 + 4;
 #pragma unroll
                     for (int q = 0; q < 3; ++q)
