@@ -155,10 +155,7 @@ FlagP flags_for(dba_ctx* c, long s)
     f.stats = c->stats;
     f.tlist = c->tlist;
     f.tctr = c->tctr;
-    if (c->den3_list) {
-        f.tctr = c->tctr + s % 2;
-        f.tctr_nxt = c->tctr + (s + 1) % 2;
-    }
+    if (c->den3_list) f.tctr = c->tctr + s % 2;
     return f;
 }
 
@@ -261,14 +258,27 @@ KHTileP<R> kh_tile_params(dba_ctx* c, bool dba_mode, long s)
     P.gmax_clear = c->kgmax + (s + 1) % 3;
     P.time = c->ktime;
     P.Kc = kh_consts<R>(k.dt, P.dx, P.dy, P.vol, P.gamma);
-    if (c->kh_full && !P.conserved) {   // (the conserved step's per-block sums live in the tile kernel)
-        P.full = c->kh_full;
-        P.hit = c->kh_hit;
-        P.cnt_prev = c->kh_cnt + (s + 2) % 3;
-        P.cnt_cur = c->kh_cnt + s % 3;
-        P.cnt_next = c->kh_cnt + (s + 1) % 3;
-    }
     return P;
+}
+
+// strips of step s, false without them (the conserved step's per-block sums live in the tile kernel)
+bool kh_strip_params(dba_ctx* c, bool dba_mode, long s, KHStripP& X)
+{
+    if (!c->kh_full || (c->cfg.conserved && dba_mode)) return false;
+    X.full = c->kh_full;
+    X.hit = c->kh_hit;
+    X.cnt_prev = c->kh_cnt + (s + 2) % 3;
+    X.cnt_cur = c->kh_cnt + s % 3;
+    X.cnt_next = c->kh_cnt + (s + 1) % 3;
+    return true;
+}
+
+template <typename R>
+cudaError_t enqueue_kh_tile(dba_ctx* c, long s, bool dba_mode, const FlagP& f)
+{
+    KHStripP X;
+    const bool strips = kh_strip_params(c, dba_mode, s, X);
+    return launch_kh_tile<R>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_tile_params<R>(c, dba_mode, s), strips ? &X : nullptr);
 }
 
 template <typename R>
@@ -338,9 +348,8 @@ cudaError_t enqueue_step_t(dba_ctx* c, long s, bool dba_mode)
     }
     case DBA_MODEL_KH: {
         if (c->kh_tiles) {
-            const KHTileP<R> T = kh_tile_params<R>(c, dba_mode, s);
-            e = launch_kh_tile<R>(c->B, dba_mode, c->grid, c->st, c->g, f, T);
-            if (e != cudaSuccess || !T.conserved) return e;
+            e = enqueue_kh_tile<R>(c, s, dba_mode, f);
+            if (e != cudaSuccess || !(c->cfg.conserved && dba_mode)) return e;
             break;
         }
         KHP<R> P = kh_params<R>(c, dba_mode);
@@ -1359,7 +1368,7 @@ int dba_step_profiled(dba_ctx* c, int nsteps, int mode, dba_prof* out)
                 }
                 else {
                     r = cudaMemsetAsync(c->count, 0, sizeof(int), c->st);
-                    if (c->kh_tiles) r = launch_kh_tile<double>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_tile_params<double>(c, dba_mode, s));
+                    if (c->kh_tiles) r = enqueue_kh_tile<double>(c, s, dba_mode, f);
                     else if (r == cudaSuccess) r = launch_kh<double>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_params<double>(c, dba_mode));
                 }
             } else {
@@ -1373,7 +1382,7 @@ int dba_step_profiled(dba_ctx* c, int nsteps, int mode, dba_prof* out)
                 }
                 else {
                     r = cudaMemsetAsync(c->count, 0, sizeof(int), c->st);
-                    if (c->kh_tiles) r = launch_kh_tile<float>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_tile_params<float>(c, dba_mode, s));
+                    if (c->kh_tiles) r = enqueue_kh_tile<float>(c, s, dba_mode, f);
                     else if (r == cudaSuccess) r = launch_kh<float>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_params<float>(c, dba_mode));
                 }
             }

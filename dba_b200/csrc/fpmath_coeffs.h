@@ -23,38 +23,8 @@
 #define DBA_FM_HD inline
 #endif
 #endif
-#ifdef __CUDACC__
-static __constant__ double dba_fm_exp_poly_c[12] = {
-    1.608665004457821e-10,
-    2.0918170876658783e-09,
-    2.5052071034565116e-08,
-    2.755726318947621e-07,
-    2.7557319247274564e-06,
-    2.4801587336526005e-05,
-    0.0001984126984126328,
-    0.0013888888888879043,
-    0.008333333333333333,
-    0.04166666666666668,
-    0.16666666666666666,
-    0.5,
-};
-#endif
 static DBA_FM_HD double dba_fm_exp_poly(double x)
 {
-#ifdef __CUDA_ARCH__
-    double p = dba_fm_exp_poly_c[0];
-    p = fma(p, x, dba_fm_exp_poly_c[1]);
-    p = fma(p, x, dba_fm_exp_poly_c[2]);
-    p = fma(p, x, dba_fm_exp_poly_c[3]);
-    p = fma(p, x, dba_fm_exp_poly_c[4]);
-    p = fma(p, x, dba_fm_exp_poly_c[5]);
-    p = fma(p, x, dba_fm_exp_poly_c[6]);
-    p = fma(p, x, dba_fm_exp_poly_c[7]);
-    p = fma(p, x, dba_fm_exp_poly_c[8]);
-    p = fma(p, x, dba_fm_exp_poly_c[9]);
-    p = fma(p, x, dba_fm_exp_poly_c[10]);
-    p = fma(p, x, dba_fm_exp_poly_c[11]);
-#else
     double p = 1.608665004457821e-10;
     p = fma(p, x, 2.0918170876658783e-09);
     p = fma(p, x, 2.5052071034565116e-08);
@@ -67,35 +37,10 @@ static DBA_FM_HD double dba_fm_exp_poly(double x)
     p = fma(p, x, 0.04166666666666668);
     p = fma(p, x, 0.16666666666666666);
     p = fma(p, x, 0.5);
-#endif
     return p;
 }
-#ifdef __CUDACC__
-static __constant__ double dba_fm_log_poly_c[9] = {
-    0.1188345239410786,
-    0.11687962997542156,
-    0.13335645841949378,
-    0.15384574966460907,
-    0.18181818595769064,
-    0.22222222219844232,
-    0.2857142857143541,
-    0.3999999999999999,
-    0.6666666666666666,
-};
-#endif
 static DBA_FM_HD double dba_fm_log_poly(double x)
 {
-#ifdef __CUDA_ARCH__
-    double p = dba_fm_log_poly_c[0];
-    p = fma(p, x, dba_fm_log_poly_c[1]);
-    p = fma(p, x, dba_fm_log_poly_c[2]);
-    p = fma(p, x, dba_fm_log_poly_c[3]);
-    p = fma(p, x, dba_fm_log_poly_c[4]);
-    p = fma(p, x, dba_fm_log_poly_c[5]);
-    p = fma(p, x, dba_fm_log_poly_c[6]);
-    p = fma(p, x, dba_fm_log_poly_c[7]);
-    p = fma(p, x, dba_fm_log_poly_c[8]);
-#else
     double p = 0.1188345239410786;
     p = fma(p, x, 0.11687962997542156);
     p = fma(p, x, 0.13335645841949378);
@@ -105,43 +50,10 @@ static DBA_FM_HD double dba_fm_log_poly(double x)
     p = fma(p, x, 0.2857142857143541);
     p = fma(p, x, 0.3999999999999999);
     p = fma(p, x, 0.6666666666666666);
-#endif
     return p;
 }
-#ifdef __CUDACC__
-static __constant__ double dba_fm_atan_poly_c[13] = {
-    -0.013905374533113234,
-    0.030622995553735516,
-    -0.04103887546862687,
-    0.04719259188242093,
-    -0.05258020272656758,
-    0.058819230561140225,
-    -0.06666641869131183,
-    0.07692306729194896,
-    -0.0909090906681608,
-    0.11111111110751482,
-    -0.1428571428571149,
-    0.19999999999999993,
-    -0.3333333333333333,
-};
-#endif
 static DBA_FM_HD double dba_fm_atan_poly(double x)
 {
-#ifdef __CUDA_ARCH__
-    double p = dba_fm_atan_poly_c[0];
-    p = fma(p, x, dba_fm_atan_poly_c[1]);
-    p = fma(p, x, dba_fm_atan_poly_c[2]);
-    p = fma(p, x, dba_fm_atan_poly_c[3]);
-    p = fma(p, x, dba_fm_atan_poly_c[4]);
-    p = fma(p, x, dba_fm_atan_poly_c[5]);
-    p = fma(p, x, dba_fm_atan_poly_c[6]);
-    p = fma(p, x, dba_fm_atan_poly_c[7]);
-    p = fma(p, x, dba_fm_atan_poly_c[8]);
-    p = fma(p, x, dba_fm_atan_poly_c[9]);
-    p = fma(p, x, dba_fm_atan_poly_c[10]);
-    p = fma(p, x, dba_fm_atan_poly_c[11]);
-    p = fma(p, x, dba_fm_atan_poly_c[12]);
-#else
     double p = -0.013905374533113234;
     p = fma(p, x, 0.030622995553735516);
     p = fma(p, x, -0.04103887546862687);
@@ -155,7 +67,6 @@ static DBA_FM_HD double dba_fm_atan_poly(double x)
     p = fma(p, x, -0.1428571428571149);
     p = fma(p, x, 0.19999999999999993);
     p = fma(p, x, -0.3333333333333333);
-#endif
     return p;
 }
 static DBA_FM_HD float dba_fm_atanf_poly(float x)

@@ -73,18 +73,14 @@ def main():
     pio2f_hi = struct.unpack("f", struct.pack("f", float(mp.pi / 2)))[0]
     pio2f_lo = struct.unpack("f", struct.pack("f", float(mp.pi / 2 - mp.mpf(pio2f_hi))))[0]
 
-    # the device reads the coefficients from the constant bank, an operand of its FP64
-    # instructions; as literals each would take two moves (the values and the result's
-    # bits are the same)
+    # literals: from __constant__ arrays the kernels were no faster, and every launch of a library with
+    # such arrays took 0.1 to 0.2 us more (7.50 -> 7.63 us per step of one launch)
     def horner(name, cs):
-        lines = ["#ifdef __CUDACC__", f"static __constant__ double {name}_c[{len(cs)}] = {{"]
-        lines += [f"    {c!r}," for c in cs]
-        lines += ["};", "#endif", f"static DBA_FM_HD double {name}(double x)", "{", "#ifdef __CUDA_ARCH__",
-                  f"    double p = {name}_c[0];"]
-        lines += [f"    p = fma(p, x, {name}_c[{k}]);" for k in range(1, len(cs))]
-        lines += ["#else", f"    double p = {cs[0]!r};"]
-        lines += [f"    p = fma(p, x, {c!r});" for c in cs[1:]]
-        lines += ["#endif", "    return p;", "}"]
+        lines = [f"static DBA_FM_HD double {name}(double x)", "{", f"    double p = {cs[0]!r};"]
+        for c in cs[1:]:
+            lines.append(f"    p = fma(p, x, {c!r});")
+        lines.append("    return p;")
+        lines.append("}")
         return "\n".join(lines)
 
     def hornerf(name, cs):

@@ -50,8 +50,9 @@ struct FlagP {
     // listed tiles of the step, for the tile kernels that hand tiles out dynamically
     // (tile_list_append / tile_queue_done); null elsewhere
     int* tlist = nullptr;       // (tile, meta) pairs
-    unsigned* tctr = nullptr;   // [0] entries listed, [1] entries taken, [2] CTAs done
-    unsigned* tctr_nxt = nullptr;   // k_dendrite3.cuh: tctr is this step's count alone, this the next step's
+    // [0] entries listed, [1] entries taken, [2] CTAs done; k_dendrite3.cuh: one of an aligned pair of
+    // counts, the step's own, the other the next step's
+    unsigned* tctr = nullptr;
 };
 
 __device__ __forceinline__ int wrapc(int v, int n, int bc)

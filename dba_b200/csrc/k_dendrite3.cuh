@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(256, Den3<R, B>::MINB) dendrite3_step(GridP g,
     const int tid = threadIdx.x, nb = g.nb, w = tid >> 5;
     __shared__ uint4 s_mask;
     const int cnt = LIST ? (int)min(__ldcg(f.tctr), (unsigned)ntiles) : ntiles;
-    if (LIST && blockIdx.x == 0 && tid == 0) *f.tctr_nxt = 0u;   // the next step's count
+    if (LIST && blockIdx.x == 0 && tid == 0)             // the next step's count: the other of the pair
+        *reinterpret_cast<unsigned*>(reinterpret_cast<uintptr_t>(f.tctr) ^ sizeof(unsigned)) = 0u;
 
     for (int i = blockIdx.x, it = 0; i < cnt; i += gridDim.x, it ^= 1) {
         int4 ea, eb;

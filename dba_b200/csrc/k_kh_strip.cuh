@@ -48,7 +48,7 @@ struct KHStrip {
 // 120 / 79, 97 % 120 / 100, 90 % 116 / 107, 81 % 106 / 110, 63 % 86 / 111; 1024^2: every
 // block 39.5 / 33, 97 % 37.6 / 48.5.  Unused, their two launches and the scan's look at the
 // neighbours cost 5 us.
-// (cnt: P.cnt_prev; before kh_strip_step clears it, P.cnt_next still holds the count that the
+// (cnt: X.cnt_prev; before kh_strip_step clears it, X.cnt_next still holds the count that the
 // step before decided by.  A restored state starts with counts of all ones: strips on.)
 __device__ __forceinline__ bool kh_strips_on(const GridP& g, const unsigned* cnt)
 {
@@ -136,7 +136,7 @@ __device__ __forceinline__ bool kh_around(const GridP& g, const uint8_t* w, int 
 }
 
 template <int B, bool DBA>
-__global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<float> P)
+__global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
 {
     constexpr int T = 16, TB = T / B, NBT = TB * TB;
     const int ntx = g.nx / T, nty = g.ny / T, ntiles = ntx * nty;
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
         if (DBA) {
             // (wake_clr holds the flags of the step before until kh_tile_step clears it)
             around = kh_around(g, f.wake_cur, bx, by);
-            if (!act && f.wake_clr[b] && kh_strips_on(g, P.cnt_next) && kh_around(g, f.wake_clr, bx, by)) s_blk[atomicAdd(&s_cnt, 1)] = b;
+            if (!act && f.wake_clr[b] && kh_strips_on(g, X.cnt_next) && kh_around(g, f.wake_clr, bx, by)) s_blk[atomicAdd(&s_cnt, 1)] = b;
         } else {
             f.wake_clr[b] = 0;
             f.wake_nxt[b] = 1;
@@ -173,12 +173,12 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
     const int g0 = (threadIdx.x & 31) & ~(NBT - 1);
     constexpr unsigned gm = (1u << NBT) - 1u;
     const unsigned abits = (ma >> g0) & gm, pbits = (mp >> g0) & gm;
-    const bool whole = ((mr >> g0) & gm) == gm, full = whole && (!DBA || kh_strips_on(g, P.cnt_prev));
+    const bool whole = ((mr >> g0) & gm) == gm, full = whole && (!DBA || kh_strips_on(g, X.cnt_prev));
     const unsigned nw = __popc(__ballot_sync(0xffffffffu, valid && kq == 0 && whole));
-    if ((threadIdx.x & 31) == 0 && nw) atomicAdd(P.cnt_cur, nw);
+    if ((threadIdx.x & 31) == 0 && nw) atomicAdd(X.cnt_cur, nw);
     unsigned vm = 0u;
     if (valid) {
-        if (kq == 0) P.full[tile] = full;
+        if (kq == 0) X.full[tile] = full;
         if (cfl) {
             if (full) P.vmax[b] = 0.f;                   // kh_strip_step takes the maximum into it
             else if (!act) vm = __float_as_uint(P.vmax[b]);
@@ -318,10 +318,10 @@ __device__ __forceinline__ void kh_pair_flux(const KHPairK& K, const Pair4& L, c
 }
 
 template <int B, bool DBA>
-__global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f, KHTileP<float> P, KHPairK K, int H)
+__global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f, KHTileP<float> P, KHStripP X, KHPairK K, int H)
 {
     constexpr int OUT = KHStrip::OUT;
-    if (DBA && blockIdx.x > 0 && !kh_strips_on(g, P.cnt_prev)) return;
+    if (DBA && blockIdx.x > 0 && !kh_strips_on(g, X.cnt_prev)) return;
     const int lane = threadIdx.x & 31;
     const int nsx = (g.nx + OUT - 1) / OUT;
     const int u = blockIdx.x * (KHStrip::NT / 32) + (threadIdx.x >> 5);
@@ -335,14 +335,14 @@ __global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f
         mh = f2_pack(-Kd.hdt, -Kd.hdt);
         dtdx = f2_pack(Kd.dtdx, Kd.dtdx);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *P.cnt_next = 0u;
+            *X.cnt_next = 0u;
             if (cfl) {
                 *P.gmax_clear = 0u;
                 *P.time += dt;
             }
         }
     }
-    if (y0 >= g.ny || (DBA && !kh_strips_on(g, P.cnt_prev))) return;
+    if (y0 >= g.ny || (DBA && !kh_strips_on(g, X.cnt_prev))) return;
     const int xr = sx * OUT + 2 * lane - 2;              // the lane's first column; past the grid's last one it is no output
     const bool own = lane >= 1 && lane <= 30 && xr < g.nx;
     int x = wrap_p(xr, g.nx);
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f
     const size_t nx = (size_t)g.nx;
     if (DBA) {                                           // a unit without a full tile has nothing to do
         bool any = false;
-        for (int y = y0; y < y0 + rows; y += 16) any |= own && P.full[x / 16 + ntx * (y / 16)];
+        for (int y = y0; y < y0 + rows; y += 16) any |= own && X.full[x / 16 + ntx * (y / 16)];
         if (!__any_sync(0xffffffffu, any)) return;
     }
 
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f
                 // update of row y - 1
                 const int yr = y - 1;
                 const int b = x / B + g.nbx * (yr / B);
-                if (yr % B == 0) on = own && (!DBA || P.full[x / 16 + ntx * (yr / 16)]);
+                if (yr % B == 0) on = own && (!DBA || X.full[x / 16 + ntx * (yr / 16)]);
                 if (on) {
                     const size_t gi = (size_t)x + nx * yr;
                     auto upd = [&](int q, f2 o, f2 d, f2 a, f2 c) -> f2 {   // field q: old value, x flux difference, fluxes above and below
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f
                         vblk = 0u;
                     }
                     if (DBA) {
-                        if (on && hit) P.hit[b] = 1;
+                        if (on && hit) X.hit[b] = 1;
                         hit = false;
                     }
                 }

@@ -72,14 +72,21 @@ struct KHTileP {
     // the formula constants (kh_consts) computed on the host, read by the kernel from the
     // parameter space; hdt and dtdx are replaced in the kernel by those of the step's dt
     KHK<R> Kc;
-    // k_kh_strip.cuh (null: no strips).  full[tile]: every block of the 16^2 tile and around it is
-    // active this step; hit[block]: a cell of a full tile's block passes the wake-up test (zero
-    // between steps)
+};
+
+// What the strips (k_kh_strip.cuh) share with the tile kernel beside them: full[tile], every block
+// of the 16^2 tile and around it is active this step; hit[block], a cell of a full tile's block
+// passes the wake-up test (zero between steps); full tiles of the step before, of this one, and
+// the word the next step counts into.
+struct KHStripP {
+    static constexpr bool on = true;
     uint8_t* full = nullptr;
     uint8_t* hit = nullptr;
-    // full tiles of the step before, of this one, and the word the next step counts into
     const unsigned* cnt_prev = nullptr;
     unsigned *cnt_cur = nullptr, *cnt_next = nullptr;
+};
+struct KHNoStrips {
+    static constexpr bool on = false;
 };
 
 // largest signal speed of a cell: sound speed + flow speed
@@ -223,8 +230,10 @@ __global__ void __launch_bounds__(256) kh_tile_scan(GridP g, FlagP f, KHTileP<R>
     }
 }
 
-template <typename R, int B, bool DBA>
-__global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_step(GridP g, FlagP f, KHTileP<R> P)
+// X: KHStripP beside strips, KHNoStrips alone (a parameter of the kernel, not a test in it: the extra
+// code costs the plain kernel 2 to 5 % in spilled registers)
+template <typename R, int B, bool DBA, typename X>
+__global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_step(GridP g, FlagP f, KHTileP<R> P, X strips)
 {
     using S = KHTile<R, B>;
     constexpr int NT = S::NT, T = S::T, TB = S::TB, NBT = S::NBT, RB = S::RB, GT = S::GT;
@@ -262,7 +271,7 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
         double dt = P.dt;
         if (cfl) {
             dt = P.cfl * P.hmin / (double)__uint_as_float(*P.gmax_prev);
-            if (blockIdx.x == 0 && !P.full) {            // (kh_strip_step does it where it runs)
+            if (!X::on && blockIdx.x == 0) {             // (kh_strip_step does it where it runs)
                 *P.gmax_clear = 0u;
                 *P.time += dt;
             }
@@ -640,23 +649,21 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
     if (i > 0) tile_end(i - 1);
     __syncthreads();
     if (cfl && tid == 0) atomicMax(P.gmax_cur, s_vcta);
-    if constexpr (DBA && sizeof(R) == 4) {
-        if (P.full) {
-            // beside strips (k_kh_strip.cuh): the flags of the step before are cleared here, and the
-            // blocks of full tiles get their next flags and wake their neighbours
-            for (int b = blockIdx.x * NT + tid; b < g.nb; b += gridDim.x * NT) {
-                f.wake_clr[b] = 0;
-                const int bx = b % g.nbx, by = b / g.nbx;
-                if (!P.full[bx / TB + ntx * (by / TB)]) continue;
-                const int h = P.hit[b];
-                f.next[b] = (uint8_t)h;
-                if (!h) continue;
-                P.hit[b] = 0;
-                const int xm = (bx == 0 ? g.nbx : bx) - 1, xp = bx + 1 == g.nbx ? 0 : bx + 1;
-                const int ym = ((by == 0 ? g.nby : by) - 1) * g.nbx, yp = (by + 1 == g.nby ? 0 : by + 1) * g.nbx, yc = by * g.nbx;
-                uint8_t* w = f.wake_nxt;
-                w[xm + ym] = w[bx + ym] = w[xp + ym] = w[xm + yc] = w[b] = w[xp + yc] = w[xm + yp] = w[bx + yp] = w[xp + yp] = 1;
-            }
+    if constexpr (DBA && X::on) {
+        // the flags of the step before are cleared here, and the blocks of full tiles get their next
+        // flags and wake their neighbours
+        for (int b = blockIdx.x * NT + tid; b < g.nb; b += gridDim.x * NT) {
+            f.wake_clr[b] = 0;
+            const int bx = b % g.nbx, by = b / g.nbx;
+            if (!strips.full[bx / TB + ntx * (by / TB)]) continue;
+            const int h = strips.hit[b];
+            f.next[b] = (uint8_t)h;
+            if (!h) continue;
+            strips.hit[b] = 0;
+            const int xm = (bx == 0 ? g.nbx : bx) - 1, xp = bx + 1 == g.nbx ? 0 : bx + 1;
+            const int ym = ((by == 0 ? g.nby : by) - 1) * g.nbx, yp = (by + 1 == g.nby ? 0 : by + 1) * g.nbx, yc = by * g.nbx;
+            uint8_t* w = f.wake_nxt;
+            w[xm + ym] = w[bx + ym] = w[xp + ym] = w[xm + yc] = w[b] = w[xp + yc] = w[xm + yp] = w[bx + yp] = w[xp + yp] = 1;
         }
     }
     if (tid == GT) tile_queue_done(f);
