@@ -55,7 +55,7 @@ struct BatchBlk {
     long long off[4];   // first halo cell west, east, south, north
     int nbr[4];         // global ids of the blocks holding those halo lines
     int meta;           // act | p parity << 2 | T parity << 3
-    int lb;             // block id within the slot
+    int lb, bx, by;     // block id and coordinates within the slot
 };
 
 // shared memory of one step of the batch kernels
@@ -154,6 +154,8 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
                 d.r = r;
                 d.meta = m & 15;
                 d.lb = lb;
+                d.bx = bx;
+                d.by = by;
                 d.gi0 = x0 + (long long)r.nx * y0;
                 d.off[0] = xw + (long long)r.nx * y0;
                 d.off[1] = xe + (long long)r.nx * y0;
@@ -238,22 +240,27 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
                 }
             }
             __syncthreads();
-            // ---- next flags and neighbour wake-up, one thread per block
-            if (DBA && tid < nk) {
-                const BatchBlk& d = s_d[tid];
-                GridP lg;
-                lg.nx = d.r.nx; lg.ny = d.r.ny; lg.nz = 1;
-                lg.nbx = d.r.nbx; lg.nby = d.r.nby; lg.nbz = 1; lg.nb = d.r.nb; lg.bc = d.r.bc;
-                const int blk = d.r.boff + d.lb;
-                if (d.meta & 1) {
-                    f.next[blk] = (uint8_t)s_np[tid];
-                    if (s_np[tid]) wake_faces(lg, f.wake_nxt + d.r.boff, d.lb);
+            // ---- next flags and neighbour wake-up (self + 4 faces; the z faces of one block layer are the
+            // block itself), one neighbour per thread from the block's coordinates.  One thread per
+            // block, working out seven neighbours of two channels with divisions, was the longest
+            // stretch of a round: @W@
+            if (DBA)
+                for (int i = tid; i < nk * 10; i += NT) {
+                    const int k = i / 10, q = i - 10 * k, ch = q / 5, n = q - 5 * ch;
+                    const BatchBlk& d = s_d[k];
+                    if (!((d.meta >> ch) & 1)) continue;
+                    const int hit = ch ? s_nT[k] : s_np[k];
+                    if (n == 0) f.next[(size_t)ch * nb + d.r.boff + d.lb] = (uint8_t)hit;
+                    if (!hit) continue;
+                    int bx = d.bx + (n == 1 ? -1 : (n == 2 ? 1 : 0)), by = d.by + (n == 3 ? -1 : (n == 4 ? 1 : 0));
+                    if (d.r.bc) {
+                        if (bx < 0 || bx >= d.r.nbx || by < 0 || by >= d.r.nby) continue;
+                    } else {
+                        bx = wrap_p(bx, d.r.nbx);
+                        by = wrap_p(by, d.r.nby);
+                    }
+                    f.wake_nxt[(size_t)ch * nb + d.r.boff + bx + d.r.nbx * by] = 1;
                 }
-                if (d.meta & 2) {
-                    f.next[nb + blk] = (uint8_t)s_nT[tid];
-                    if (s_nT[tid]) wake_faces(lg, f.wake_nxt + nb + d.r.boff, d.lb);
-                }
-            }
             __syncthreads();
         }
     }
