@@ -122,7 +122,8 @@ struct dba_batch {
     int esz = 4;
     int sms = 148, grid = 148;
     cudaStream_t st = nullptr;
-    void* arena = nullptr;           // 4 arrays x cell_capacity x esz
+    void* arena = nullptr;           // 4 arrays of `stride` cells
+    size_t stride = 0;               // cell_capacity rounded up
     SlotRec* d_slots = nullptr;
     int* d_bslot = nullptr;
     int* d_hi = nullptr;             // 1 + highest block id of a live slot
@@ -258,7 +259,9 @@ int dba_batch_create(const dba_batch_config* cfg, dba_batch** out)
         b->cfg.cell_capacity = cells;
     }
     const size_t NB = cfg->block_capacity;
-    if (e == cudaSuccess) e = cudaMalloc(&b->arena, 4 * cells * b->esz);
+    // (each of the four arrays starts on a 16-byte boundary, as every slot in it does)
+    b->stride = (cells + 15) / 16 * 16;
+    if (e == cudaSuccess) e = cudaMalloc(&b->arena, 4 * b->stride * b->esz);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_slots, sizeof(SlotRec) * cfg->max_slots);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_bslot, sizeof(int) * NB);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hi, sizeof(int));
@@ -331,7 +334,7 @@ int dba_batch_add(dba_batch* b, const dba_config* k, const double* ic, int* slot
         b->cells.give(coff, n);
         return DBA_ERR_NOMEM;
     }
-    const size_t cap = b->cfg.cell_capacity;
+    const size_t cap = b->stride;
     unsigned char* base = (unsigned char*)b->arena;
     SlotRec r{};
     r.nx = k->nx; r.ny = k->ny; r.nbx = nbx; r.nby = nby; r.nb = nb; r.boff = (int)boff; r.bc = k->bc; r.live = 1;

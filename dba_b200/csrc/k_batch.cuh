@@ -60,10 +60,14 @@ struct BatchBlk {
 
 // shared memory of one step of the batch kernels
 template <typename R, int B, int NT> struct BatchSmem {
-    static constexpr int TV = (B + 2) * (B + 2);
+    static constexpr int PC = 16 / (int)sizeof(R);       // cells per 16-byte piece
+    // row pitch: column x at x + PC.  Column -1 takes the last cell before a row's first piece
+    // and column B, at W, the first cell of the next row; no piece covers either
+    static constexpr int W = B + PC;
+    static constexpr int TV = W * (B + 2);
     static constexpr int K = batch_group<B, NT>();
-    R sp[K * TV];
-    R sT[K * TV];
+    alignas(16) R sp[K * TV];
+    alignas(16) R sT[K * TV];
     int s_list[NT], s_lmeta[NT];
     int s_cnt;
     int s_np[K], s_nT[K];
@@ -84,10 +88,10 @@ template <bool COHERENT, typename T> __device__ __forceinline__ T ldx(const T* p
 template <typename R, int B, int NT, bool DBA, bool COHERENT>
 __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f, BatchSmem<R, B, NT>& S)
 {
+    using M = BatchSmem<R, B, NT>;
     constexpr int V = B * B;
-    constexpr int E = B + 2;
-    constexpr int TV = E * E;
-    constexpr int K = batch_group<B, NT>();
+    constexpr int PC = M::PC, W = M::W, TV = M::TV;
+    constexpr int K = M::K;
     constexpr int CPT = K * V / NT;
     static_assert(K * V % NT == 0 && CPT >= 1, "group must give every thread whole cells");
     R* const sp = S.sp;
@@ -169,37 +173,38 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
                 s_nT[tid] = 0;
             }
             __syncthreads();
-            // ---- stage the group: interiors from the block's current buffer; each
-            // halo line from both buffers of the block holding it, selected by that
-            // block's parity loaded alongside (one round trip); corners are never read
-            for (int i = tid; i < nk * TV; i += NT) {
-                const int k = i / TV;
-                const int j = i - k * TV;
-                const int ly = j / E, lx = j - ly * E;
-                const bool ix = lx >= 1 && lx <= B, iy = ly >= 1 && ly <= B;
-                if (!ix && !iy) continue;
+            // ---- stage the group: interiors from the block's current buffer as 16-byte asynchronous
+            // pieces (through L2; a slot's arrays start on 16-byte boundaries); each halo line
+            // from both buffers of the block holding it, selected by that block's parity loaded
+            // alongside (one round trip); corners are never read.  Cell by cell, a thread of a
+            // group of 1024 cells waited for memory ten times over: 16 sims of
+            // 128..512 cells in 16^2 blocks 12.56 -> 11.12 us per step, 14 of 96..384 12.79 -> 11.16.
+            constexpr int PR = B / PC, PB = B * PR;          // pieces per row, per block and field
+            for (int i = tid; i < nk * PB; i += NT) {
+                const int k = i / PB, q = i - k * PB, ly = q / PR, c = q - ly * PR;
                 const BatchBlk& d = s_d[k];
-                const R* P0 = (const R*)d.r.p[0];
-                const R* P1 = (const R*)d.r.p[1];
-                const R* T0 = (const R*)d.r.T[0];
-                const R* T1 = (const R*)d.r.T[1];
-                R vp, vT;
-                if (ix && iy) {
-                    const long long o = d.gi0 + (lx - 1) + (long long)d.r.nx * (ly - 1);
-                    vp = ldx<COHERENT>(((d.meta & 4) ? P1 : P0) + o);
-                    vT = ldx<COHERENT>(((d.meta & 8) ? T1 : T0) + o);
-                } else {
-                    const int fc = ix ? (ly == 0 ? 2 : 3) : (lx == 0 ? 0 : 1);
-                    const long long o = d.off[fc] + (ix ? (long long)(lx - 1) : (long long)d.r.nx * (ly - 1));
-                    const int nbid = d.nbr[fc];
-                    const R a0 = ldx<COHERENT>(P0 + o), a1 = ldx<COHERENT>(P1 + o);
-                    const R c0 = ldx<COHERENT>(T0 + o), c1 = ldx<COHERENT>(T1 + o);
-                    vp = ldx<COHERENT>(f.par_cur + nbid) ? a1 : a0;
-                    vT = ldx<COHERENT>(f.par_cur + nb + nbid) ? c1 : c0;
-                }
-                sp[i] = vp;
-                sT[i] = vT;
+                const long long o = d.gi0 + PC * c + (long long)d.r.nx * ly;
+                const int so = k * TV + W * (ly + 1) + PC * (c + 1);
+                cp_async16(sp + so, (const R*)((d.meta & 4) ? d.r.p[1] : d.r.p[0]) + o);
+                cp_async16(sT + so, (const R*)((d.meta & 8) ? d.r.T[1] : d.r.T[0]) + o);
             }
+            cp_async_commit();
+            // (all of a thread's halo cells in flight at once, up to four: more would cost registers)
+            constexpr int HU = (K * 4 * B + NT - 1) / NT > 4 ? 4 : (K * 4 * B + NT - 1) / NT;
+#pragma unroll HU
+            for (int i = tid; i < nk * 4 * B; i += NT) {
+                const int k = i / (4 * B), q = i - k * 4 * B, fc = q / B, e = q - fc * B;   // face (W, E, S, N), cell on it
+                const BatchBlk& d = s_d[k];
+                const long long o = d.off[fc] + (fc < 2 ? (long long)d.r.nx * e : (long long)e);
+                const int nbid = d.nbr[fc];
+                const R a0 = ldx<COHERENT>((const R*)d.r.p[0] + o), a1 = ldx<COHERENT>((const R*)d.r.p[1] + o);
+                const R c0 = ldx<COHERENT>((const R*)d.r.T[0] + o), c1 = ldx<COHERENT>((const R*)d.r.T[1] + o);
+                const bool qp = ldx<COHERENT>(f.par_cur + nbid) != 0, qT = ldx<COHERENT>(f.par_cur + nb + nbid) != 0;
+                const int so = k * TV + (fc < 2 ? W * (e + 1) + (fc == 0 ? PC - 1 : PC + B) : (fc == 2 ? 0 : W * (B + 1)) + PC + e);
+                sp[so] = qp ? a1 : a0;
+                sT[so] = qT ? c1 : c0;
+            }
+            cp_async_wait0();
             __syncthreads();
             // ---- advance: CPT cells per thread, cells of a block on consecutive threads
 #pragma unroll
@@ -211,16 +216,16 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
                 const BatchBlk& d = s_d[k];
                 const int m = d.meta;
                 const int ly = v / B, lx = v - ly * B;
-                const int ti = k * TV + (lx + 1) + E * (ly + 1);
+                const int ti = k * TV + lx + PC + W * (ly + 1);
                 const long long gi = d.gi0 + lx + (long long)d.r.nx * ly;
                 const R f0 = (R)d.r.f0, f1 = (R)d.r.f1, f2 = (R)d.r.f2, f3 = (R)d.r.f3, dt = (R)d.r.dt;
                 const R pc = sp[ti], Tc = sT[ti];
                 R pn = pc;
                 if (m & 1) {
                     if constexpr (std::is_same<R, float>::value)
-                        pn = den_p_f32<2>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + E], sp[ti - E], pc, pc, d.r.c32);
+                        pn = den_p_f32<2>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + W], sp[ti - W], pc, pc, d.r.c32);
                     else
-                        pn = den_p_new<R>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + E], sp[ti - E], pc, pc, f0, f1, f2,
+                        pn = den_p_new<R>(pc, Tc, sp[ti + 1], sp[ti - 1], sp[ti + W], sp[ti - W], pc, pc, f0, f1, f2,
                                           f3, dt, (R)d.r.delta, (R)d.r.eps2, (R)d.r.gamma);
                     ((m & 4) ? (R*)d.r.p[0] : (R*)d.r.p[1])[gi] = pn;
                     if (pn >= (R)d.r.thr_p && pn <= (R)d.r.thr_p_hi) s_np[k] = 1;
@@ -229,10 +234,10 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
                 if (m & 2) {
                     R Tn;
                     if constexpr (std::is_same<R, float>::value)
-                        Tn = den_T_f32<2, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + E], sT[ti - E], Tc, Tc, (m & 1) != 0,
+                        Tn = den_T_f32<2, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + W], sT[ti - W], Tc, Tc, (m & 1) != 0,
                                                pn, pc, d.r.c32);
                     else
-                        Tn = den_T_new<R, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + E], sT[ti - E], Tc, Tc,
+                        Tn = den_T_new<R, DBA>(Tc, sT[ti + 1], sT[ti - 1], sT[ti + W], sT[ti - W], Tc, Tc,
                                                (m & 1) != 0, pn, pc, f1, dt);
                     ((m & 8) ? (R*)d.r.T[0] : (R*)d.r.T[1])[gi] = Tn;
                     if (fabs(Tn - Tc) >= (R)d.r.thr_T) s_nT[k] = 1;
@@ -243,7 +248,7 @@ __device__ __forceinline__ void batch_step_body(const BatchP& bp, const FlagP& f
             // ---- next flags and neighbour wake-up (self + 4 faces; the z faces of one block layer are the
             // block itself), one neighbour per thread from the block's coordinates.  One thread per
             // block, working out seven neighbours of two channels with divisions, was the longest
-            // stretch of a round: @W@
+            // stretch of a round: 7 sims of 96..384 cells in 8^2 blocks 6.93 -> 6.18 us per step.
             if (DBA)
                 for (int i = tid; i < nk * 10; i += NT) {
                     const int k = i / 10, q = i - 10 * k, ch = q / 5, n = q - 5 * ch;
