@@ -409,27 +409,32 @@ def run_ours(args, w):
     return result
 
 
+def kh_strips(w):
+    """KH workloads whose fully active tiles go by strips (FP32, 2^20 cells and more, not conserved)."""
+    return w["model"] == "kh" and w["precision"] == 1 and w["nx"] * w["ny"] >= 1 << 20 and not w["conserved"]
+
+
 def queue_path(w):
     """Workloads whose step is a scan kernel listing the step's tiles and the tile kernel that
-    takes them (KH tiles, FP32 3-D dendrite tiles)."""
+    takes them (KH tiles, large FP32 3-D dendrite grids)."""
     return w["model"] == "kh" or (w["model"] == "dendrite" and w["nz"] > 1 and w["precision"] == 1)
 
 
 def launches_per_step(w):
     """This engine's kernel launches per step."""
-    if w["model"] == "kh":   # tile scan + tile kernel (grids of 16-cell multiples, blocks 8 or 16)
-        return 2 + (2 if w["conserved"] else 0)
+    if w["model"] == "kh":   # tile scan + (strips) + tile kernel (grids of 16-cell multiples, blocks 8 or 16)
+        return (3 if kh_strips(w) and w["mode"] else 2) + (2 if w["conserved"] else 0)
     if queue_path(w):
         return 2
-    if w["model"] == "modelb" and w["conserved"] and not (w["precision"] == 1 and w["nz"] == 1):
-        return 3   # FP64 / 3-D conserved: step, reduce, correct
-    return 1       # FP32 2-D conserved Model B: the reduction is inside the step kernel
+    if w["model"] == "modelb" and not (w["precision"] == 1 and w["nz"] == 1):
+        return 2 + (2 if w["conserved"] else 0)   # FP64 / 3-D: potentials, update (reduce, correct)
+    return 1       # FP32 2-D Model B: one kernel, the conserved reduction inside it
 
 
 def step_is_stencil(w):
-    """The step is the stencil kernel alone (with its tile scan where it has one): no separate
+    """The step is stencil kernels alone (with a tile scan where it has one): no separate
     conserved reduction and correction launches."""
-    return launches_per_step(w) == (2 if queue_path(w) else 1)
+    return not w["conserved"] or (w["model"] == "modelb" and w["precision"] == 1 and w["nz"] == 1)
 
 
 def _ref_input(w, nx, ny):

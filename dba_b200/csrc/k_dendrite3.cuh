@@ -1,7 +1,7 @@
 // k_dendrite3.cuh -- 3-D dendrite step over tiles of 32 x 8 x 8 cells: FP64, FP32 in 4^3 blocks,
 // and small FP32 grids in 8^3 blocks (large ones: k_dendrite_tile.cuh).
 //
-// Same DBA semantics and point arithmetic as dendrite_step (k_dendrite.cuh).  A scan kernel
+// Same DBA semantics as every dendrite kernel; point arithmetic in k_dendrite.cuh.  A scan kernel
 // does the step's block bookkeeping and lists the tiles that have an active block, with
 // their blocks' activity and parity; the CTAs of the tile kernel, a few times as many as
 // are resident, step through the list (small grids: no list, a CTA per tile).  Per tile:

@@ -1,7 +1,7 @@
 // k_dendrite_tile.cuh -- FP32 3-D dendrite step over 32x8x8-cell tiles.
 //
-// Same DBA semantics and the same point arithmetic as dendrite_step
-// (k_dendrite.cuh; den_p_f32 / den_T_f32 fix every rounding) for 8^3 blocks,
+// Same DBA semantics and the same point arithmetic as the other dendrite
+// kernels (k_dendrite.cuh; den_p_f32 / den_T_f32 fix every rounding) for 8^3 blocks,
 // reorganised so that a CTA works on four x-adjacent blocks at a time:
 //
 //   * a tile is listed when any channel (p or T) of any of its blocks is

@@ -1,6 +1,6 @@
 // k_modelb_fast.cuh -- FP32 2-D Model B step (the throughput path).
 //
-// Same DBA semantics as modelb_step (k_modelb.cuh): potentials recomputed for
+// Same DBA semantics as modelb_mu / modelb_update (k_modelb.cuh): potentials recomputed for
 // halo cells whose block is active, persisted (stale) potentials read where it
 // is not, per-block ping-pong buffers.  What changes for speed:
 //   * staging looks up owner parity (and conserved offset) once per neighbour

@@ -88,7 +88,8 @@ typedef struct dba_config {
     int ic_corner;             /* dendrite tanh seed at cell (0,0,0) instead of the centre */
     double noise_amp, noise_amp_z; /* Model B: x,y and z uniform-noise amplitudes (0.05, 0.001) */
     int tiles;                 /* 1 (default): tile kernels where the shape allows -- FP32 2-D Model B on 32x32
-                                  cells (block 8, 16 or 32; nx, ny multiples of 32, or at least 64 and 2^16 cells), KH on 16x16 cells (nx, ny
+                                  cells (block 8, 16 or 32; nx, ny multiples of 32, or at least 64
+                                  and 2^16 cells), KH on 16x16 cells (nx, ny
                                   multiples of 16, block 8 or 16), FP32 3-D dendrite on 32x8x8 cells (block 8);
                                   2: as 1, with the FP32 2-D Model B tiles staged by
                                   bulk copies of the TMA engine (one per block segment of a staged row)
