@@ -121,10 +121,16 @@ void* work_alloc(dba_ctx* c, size_t bytes, int* err)
     return p;
 }
 
-// the state was replaced: no list or count of the step before it is valid
-int reset_work(dba_ctx* c)
+// The state was replaced: no list or count of the step before it is valid.  Strips: the next step
+// uses them (its cnt_prev is all ones); the step before left no ring to persist, or (pending)
+// may have (its cnt_next is all ones too).
+int reset_work(dba_ctx* c, bool pending = false)
 {
-    if (c->kh_cnt) DBA_TRY(cudaMemsetAsync(c->kh_cnt, 0xff, 3 * sizeof(unsigned), c->st));
+    if (c->kh_cnt) {
+        DBA_TRY(cudaMemsetAsync(c->kh_cnt, 0, 3 * sizeof(unsigned), c->st));
+        DBA_TRY(cudaMemsetAsync(c->kh_cnt + c->step % 3, 0xff, sizeof(unsigned), c->st));
+        if (pending) DBA_TRY(cudaMemsetAsync(c->kh_cnt + (c->step + 2) % 3, 0xff, sizeof(unsigned), c->st));
+    }
     return c->den3_list ? cuda_status(cudaMemsetAsync(c->tctr, 0, 4 * sizeof(unsigned), c->st)) : DBA_OK;
 }
 
@@ -271,6 +277,16 @@ bool kh_strip_params(dba_ctx* c, bool dba_mode, long s, KHStripP& X)
     X.cnt_cur = c->kh_cnt + s % 3;
     X.cnt_next = c->kh_cnt + (s + 1) % 3;
     return true;
+}
+
+// Before a save: what the strips of the last step left for the next step's scan to persist goes
+// into the state now, computed with the constants that step took
+int flush_rings(dba_ctx* c)
+{
+    KHStripP X;
+    const long s = c->step + 1;
+    if (!c->initialized || !kh_strip_params(c, true, s, X)) return DBA_OK;
+    return cuda_status(launch_kh_strip_flush(c->B, c->st, c->g, flags_for(c, s), kh_tile_params<float>(c, true, s), X));
 }
 
 template <typename R>
@@ -1444,6 +1460,8 @@ int dba_save_state(dba_ctx* c, void* host, size_t size)
     size_t need = 0;
     dba_state_size(c, &need);
     if (size < need) return DBA_ERR_ARG;
+    const int st = flush_rings(c);
+    if (st) return st;
     unsigned char* h = (unsigned char*)host;
     std::memcpy(h, &c->step, sizeof(long));
     std::memcpy(h + sizeof(long), &c->time, sizeof(double));
@@ -1486,6 +1504,8 @@ int dba_checkpoint(dba_ctx* c, const char* path)
 {
     if (!c || !path) return DBA_ERR_ARG;
     if (!c->initialized) return DBA_ERR_STATE;
+    const int st = flush_rings(c);
+    if (st) return st;
     DBA_TRY(cudaStreamSynchronize(c->st));
     FILE* f = std::fopen(path, "wb");
     if (!f) return DBA_ERR_IO;
@@ -1542,7 +1562,10 @@ int dba_restore(dba_ctx* c, const char* path)
     c->step = step;
     c->time = time;
     c->initialized = true;
-    return reset_work(c);
+    // a file may have been written without the rings of the blocks that fell asleep in its last step
+    // (checkpoints flush them now); with the same constants, computing them again is exact
+    const dba_config &a = cfg, &b = c->cfg;
+    return reset_work(c, a.dt == b.dt && a.cfl == b.cfl && a.dx == b.dx && a.dy == b.dy && a.kh_gamma == b.kh_gamma);
 }
 
 int dba_tip_profile(dba_ctx* c, int field, int dz, int* tip_x, int* tip_x_max)

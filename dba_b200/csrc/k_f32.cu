@@ -17,6 +17,14 @@ cudaError_t launch_gather_lazy(cudaStream_t st, const GridP& g, int B, const flo
     return cudaGetLastError();
 }
 
+cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P, const KHStripP& X)
+{
+    const int grid = (g.nb + 255) / 256;
+    if (B == 8) kh_strip_flush<8><<<grid, 256, 0, st>>>(g, f, P, X);
+    else kh_strip_flush<16><<<grid, 256, 0, st>>>(g, f, P, X);
+    return cudaGetLastError();
+}
+
 bool modelb_tiles_ok(int D, int B, int nx, int ny)
 {
     // Grids of whole tiles; or of whole blocks, two tiles across and 64 tiles in all: the last tiles

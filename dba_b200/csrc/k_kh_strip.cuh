@@ -49,7 +49,8 @@ struct KHStrip {
 // block 39.5 / 33, 97 % 37.6 / 48.5.  Unused, their two launches and the scan's look at the
 // neighbours cost 5 us.
 // (cnt: X.cnt_prev; before kh_strip_step clears it, X.cnt_next still holds the count that the
-// step before decided by.  A restored state starts with counts of all ones: strips on.)
+// step before decided by.  After a load cnt_prev is all ones (strips on) and the others are zero: the
+// state's rings are complete.)
 __device__ __forceinline__ bool kh_strips_on(const GridP& g, const unsigned* cnt)
 {
     const unsigned n = (unsigned)((g.nx / 16) * (g.ny / 16)), lacking = n - min(*cnt, n);
@@ -135,70 +136,10 @@ __device__ __forceinline__ bool kh_around(const GridP& g, const uint8_t* w, int 
     return w[xm + ym] && w[bx + ym] && w[xp + ym] && w[xm + yc] && w[xp + yc] && w[xm + yp] && w[bx + yp] && w[xp + yp];
 }
 
-template <int B, bool DBA>
-__global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
+// Ring persistence of `cnt` blocks that fell asleep, by the warps of a CTA of 256, half a ring each: what
+// their neighbours can read of them (kh_tile_step)
+__device__ __forceinline__ void kh_persist_rings(const GridP& g, const FlagP& f, const KHTileP<float>& P, int B, const int* s_blk, int cnt)
 {
-    constexpr int T = 16, TB = T / B, NBT = TB * TB;
-    const int ntx = g.nx / T, nty = g.ny / T, ntiles = ntx * nty;
-    const int it = blockIdx.x * 256 + threadIdx.x;       // the grid covers the blocks; a tile's on adjacent lanes
-    const int tile = it / NBT, kq = it % NBT;
-    const bool valid = tile < ntiles;
-    const int tby = tile / ntx, tbx = tile - tby * ntx;
-    const int bx = tbx * TB + kq % TB, by = tby * TB + kq / TB, b = bx + g.nbx * by;
-    const bool cfl = P.cfl > 0.0;
-    __shared__ int s_blk[256], s_cnt;                    // blocks that fell asleep since the step before
-    if (DBA) {
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-    }
-    int act = 0, pp = 0;
-    bool around = true;                                  // the blocks around this one are active
-    if (valid) {
-        pp = f.par_cur[b];
-        act = DBA ? (f.wake_cur[b] ? 1 : 0) : 1;
-        f.par_nxt[b] = (uint8_t)(pp ^ act);
-        if (DBA) {
-            // (wake_clr holds the flags of the step before until kh_tile_step clears it)
-            around = kh_around(g, f.wake_cur, bx, by);
-            if (!act && f.wake_clr[b] && kh_strips_on(g, X.cnt_next) && kh_around(g, f.wake_clr, bx, by)) s_blk[atomicAdd(&s_cnt, 1)] = b;
-        } else {
-            f.wake_clr[b] = 0;
-            f.wake_nxt[b] = 1;
-        }
-    }
-    count_stats(f.stats, act, valid);
-    const unsigned ma = __ballot_sync(0xffffffffu, valid && act);
-    const unsigned mr = __ballot_sync(0xffffffffu, valid && act && around);
-    const unsigned mp = __ballot_sync(0xffffffffu, valid && pp);
-    const int g0 = (threadIdx.x & 31) & ~(NBT - 1);
-    constexpr unsigned gm = (1u << NBT) - 1u;
-    const unsigned abits = (ma >> g0) & gm, pbits = (mp >> g0) & gm;
-    const bool whole = ((mr >> g0) & gm) == gm, full = whole && (!DBA || kh_strips_on(g, X.cnt_prev));
-    const unsigned nw = __popc(__ballot_sync(0xffffffffu, valid && kq == 0 && whole));
-    if ((threadIdx.x & 31) == 0 && nw) atomicAdd(X.cnt_cur, nw);
-    unsigned vm = 0u;
-    if (valid) {
-        if (kq == 0) X.full[tile] = full;
-        if (cfl) {
-            if (full) P.vmax[b] = 0.f;                   // kh_strip_step takes the maximum into it
-            else if (!act) vm = __float_as_uint(P.vmax[b]);
-        }
-    }
-    if (!DBA) return;
-    const int X0 = tbx * T, Y0 = tby * T;
-    const bool inner = X0 >= 2 && X0 + T + 2 <= g.nx && Y0 >= 2 && Y0 + T + 2 <= g.ny;
-    tile_list_append(f, valid && kq == 0 && abits != 0 && !full, tbx | (tby << 15) | ((int)inner << 30),
-                     abits | (pbits << 16), (unsigned)ntiles);
-    if (cfl) {
-        vm = __reduce_max_sync(0xffffffffu, vm);
-        if ((threadIdx.x & 31) == 0 && vm) atomicMax(P.gmax_cur, vm);
-    }
-    // Ring persistence of the blocks that fell asleep, half a ring per warp: what their neighbours can
-    // read of them (kh_tile_step).  A block with an inactive neighbour in the step before was
-    // in a listed tile, whose update has persisted it.
-    __syncthreads();
-    const int cnt = s_cnt;
-    if (cnt == 0) return;
     double dt;
     const KHK<float> K = kh_strip_consts(P, P.gmax_clear, dt);   // (the maximum that gave the step before its dt)
     const int lane = threadIdx.x & 31;
@@ -232,6 +173,89 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
             }
         }
     }
+}
+
+// Whether block (bx, by), asleep in this step, has a ring to persist: it fell asleep since the step
+// before, which advanced it by strips.  (A block with an inactive neighbour then was in a listed tile,
+// whose update has persisted it; wake_clr holds the flags of that step until kh_tile_step clears it.)
+__device__ __forceinline__ bool kh_ring_pending(const GridP& g, const FlagP& f, const KHStripP& X, int b, int bx, int by)
+{
+    return f.wake_clr[b] && kh_strips_on(g, X.cnt_next) && kh_around(g, f.wake_clr, bx, by);
+}
+
+template <int B, bool DBA>
+__global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
+{
+    constexpr int T = 16, TB = T / B, NBT = TB * TB;
+    const int ntx = g.nx / T, nty = g.ny / T, ntiles = ntx * nty;
+    const int it = blockIdx.x * 256 + threadIdx.x;       // the grid covers the blocks; a tile's on adjacent lanes
+    const int tile = it / NBT, kq = it % NBT;
+    const bool valid = tile < ntiles;
+    const int tby = tile / ntx, tbx = tile - tby * ntx;
+    const int bx = tbx * TB + kq % TB, by = tby * TB + kq / TB, b = bx + g.nbx * by;
+    const bool cfl = P.cfl > 0.0;
+    __shared__ int s_blk[256], s_cnt;                    // blocks that fell asleep since the step before
+    if (DBA) {
+        if (threadIdx.x == 0) s_cnt = 0;
+        __syncthreads();
+    }
+    int act = 0, pp = 0;
+    bool around = true;                                  // the blocks around this one are active
+    if (valid) {
+        pp = f.par_cur[b];
+        act = DBA ? (f.wake_cur[b] ? 1 : 0) : 1;
+        f.par_nxt[b] = (uint8_t)(pp ^ act);
+        if (DBA) {
+            around = kh_around(g, f.wake_cur, bx, by);
+            if (!act && kh_ring_pending(g, f, X, b, bx, by)) s_blk[atomicAdd(&s_cnt, 1)] = b;
+        } else {
+            f.wake_clr[b] = 0;
+            f.wake_nxt[b] = 1;
+        }
+    }
+    count_stats(f.stats, act, valid);
+    const unsigned ma = __ballot_sync(0xffffffffu, valid && act);
+    const unsigned mr = __ballot_sync(0xffffffffu, valid && act && around);
+    const unsigned mp = __ballot_sync(0xffffffffu, valid && pp);
+    const int g0 = (threadIdx.x & 31) & ~(NBT - 1);
+    constexpr unsigned gm = (1u << NBT) - 1u;
+    const unsigned abits = (ma >> g0) & gm, pbits = (mp >> g0) & gm;
+    const bool whole = ((mr >> g0) & gm) == gm, full = whole && (!DBA || kh_strips_on(g, X.cnt_prev));
+    const unsigned nw = __popc(__ballot_sync(0xffffffffu, valid && kq == 0 && whole));
+    if ((threadIdx.x & 31) == 0 && nw) atomicAdd(X.cnt_cur, nw);
+    unsigned vm = 0u;
+    if (valid) {
+        if (kq == 0) X.full[tile] = full;
+        if (cfl) {
+            if (full) P.vmax[b] = 0.f;                   // kh_strip_step takes the maximum into it
+            else if (!act) vm = __float_as_uint(P.vmax[b]);
+        }
+    }
+    if (!DBA) return;
+    const int X0 = tbx * T, Y0 = tby * T;
+    const bool inner = X0 >= 2 && X0 + T + 2 <= g.nx && Y0 >= 2 && Y0 + T + 2 <= g.ny;
+    tile_list_append(f, valid && kq == 0 && abits != 0 && !full, tbx | (tby << 15) | ((int)inner << 30),
+                     abits | (pbits << 16), (unsigned)ntiles);
+    if (cfl) {
+        vm = __reduce_max_sync(0xffffffffu, vm);
+        if ((threadIdx.x & 31) == 0 && vm) atomicMax(P.gmax_cur, vm);
+    }
+    __syncthreads();
+    if (s_cnt) kh_persist_rings(g, f, P, B, s_blk, s_cnt);
+}
+
+// The rings that the next step's scan would persist, ahead of a save: a saved state holds them, since
+// another context that loads it may take its steps with other constants.
+template <int B>
+__global__ void __launch_bounds__(256) kh_strip_flush(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
+{
+    __shared__ int s_blk[256], s_cnt;
+    const int b = blockIdx.x * 256 + threadIdx.x;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    if (b < g.nb && !f.wake_cur[b] && kh_ring_pending(g, f, X, b, b % g.nbx, b / g.nbx)) s_blk[atomicAdd(&s_cnt, 1)] = b;
+    __syncthreads();
+    if (s_cnt) kh_persist_rings(g, f, P, B, s_blk, s_cnt);
 }
 
 // ---- the formulas on pairs of columns (k_pair.cuh): lane by lane the operations, their order

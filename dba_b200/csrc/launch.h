@@ -91,6 +91,8 @@ template <typename R> int kh_tile_grid(int B, int sms, int ntiles);
 template <typename R>
 cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
                            const KHTileP<R>& P, const KHStripP* X);   // X: null without strips
+// rings of the blocks that the next step finds asleep (k_kh_strip.cuh); f, P, X: of the next step
+cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P, const KHStripP& X);
 // out[k] = buf[par[owner(cell)]][start + k*stride] for k < count (par may be null -> buffer 0)
 template <typename R>
 cudaError_t launch_gather(cudaStream_t st, const GridP& g, int B, int D, const R* b0, const R* b1, const uint8_t* par,
