@@ -72,8 +72,8 @@ struct dba_ctx {
                                       //   larger domain (dba_slab_rows); 0: this context's cells
     int* tlist = nullptr;             // tile queue of the tile kernels that take tiles dynamically
     unsigned* tctr = nullptr;         //   (2 ints per tile; counters, zeroed by each step's last CTA)
-    uint8_t *kh_full = nullptr, *kh_hit = nullptr;   // KH strips (k_kh_strip.cuh): per tile, per block
-    unsigned* kh_cnt = nullptr;       //   [3] full tiles of a step, rotating
+    uint8_t* kh_full = nullptr;       // KH strips (k_kh_strip.cuh): per tile
+    unsigned* kh_cnt = nullptr;       //   [3] full tiles of a step, rotating; units taken
     float* kvmax = nullptr;           // KH tiles: per-block largest signal speed (CFL)
     unsigned* kgmax = nullptr;        // KH tiles: rotating maxima of the CFL speed, float bits [3]
     double* ktime = nullptr;          // KH tiles: simulated time accumulated on the device (CFL)
@@ -122,14 +122,13 @@ void* work_alloc(dba_ctx* c, size_t bytes, int* err)
 }
 
 // The state was replaced: no list or count of the step before it is valid.  Strips: the next step
-// uses them (its cnt_prev is all ones); the step before left no ring to persist, or (pending)
-// may have (its cnt_next is all ones too).
-int reset_work(dba_ctx* c, bool pending = false)
+// uses them (its cnt_prev is all ones), and the step before left no ring for it to persist.
+int reset_work(dba_ctx* c)
 {
     if (c->kh_cnt) {
+        DBA_TRY(cudaMemsetAsync(c->kh_full, 0, (size_t)(c->cfg.nx / 16) * (c->cfg.ny / 16), c->st));
         DBA_TRY(cudaMemsetAsync(c->kh_cnt, 0, 3 * sizeof(unsigned), c->st));
         DBA_TRY(cudaMemsetAsync(c->kh_cnt + c->step % 3, 0xff, sizeof(unsigned), c->st));
-        if (pending) DBA_TRY(cudaMemsetAsync(c->kh_cnt + (c->step + 2) % 3, 0xff, sizeof(unsigned), c->st));
     }
     return c->den3_list ? cuda_status(cudaMemsetAsync(c->tctr, 0, 4 * sizeof(unsigned), c->st)) : DBA_OK;
 }
@@ -272,10 +271,10 @@ bool kh_strip_params(dba_ctx* c, bool dba_mode, long s, KHStripP& X)
 {
     if (!c->kh_full || (c->cfg.conserved && dba_mode)) return false;
     X.full = c->kh_full;
-    X.hit = c->kh_hit;
     X.cnt_prev = c->kh_cnt + (s + 2) % 3;
     X.cnt_cur = c->kh_cnt + s % 3;
     X.cnt_next = c->kh_cnt + (s + 1) % 3;
+    X.taken = c->kh_cnt + 3;
     return true;
 }
 
@@ -286,7 +285,7 @@ int flush_rings(dba_ctx* c)
     KHStripP X;
     const long s = c->step + 1;
     if (!c->initialized || !kh_strip_params(c, true, s, X)) return DBA_OK;
-    return cuda_status(launch_kh_strip_flush(c->B, c->st, c->g, flags_for(c, s), kh_tile_params<float>(c, true, s), X));
+    return cuda_status(launch_kh_strip_flush(c->B, c->st, c->g, flags_for(c, s), kh_tile_params<float>(c, true, s)));
 }
 
 template <typename R>
@@ -294,7 +293,7 @@ cudaError_t enqueue_kh_tile(dba_ctx* c, long s, bool dba_mode, const FlagP& f)
 {
     KHStripP X;
     const bool strips = kh_strip_params(c, dba_mode, s, X);
-    return launch_kh_tile<R>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_tile_params<R>(c, dba_mode, s), strips ? &X : nullptr);
+    return launch_kh_tile<R>(c->B, dba_mode, c->grid, c->st, c->g, f, kh_tile_params<R>(c, dba_mode, s), strips ? &X : nullptr, c->sms);
 }
 
 template <typename R>
@@ -815,8 +814,7 @@ int dba_create(const dba_config* cfg, dba_ctx** out)
         if (!err) c->tctr = (unsigned*)dev_alloc(c, 4 * sizeof(unsigned), &err);
         if (!err && kh_strips_ok(c->esz, cfg->nx, cfg->ny)) {
             c->kh_full = (uint8_t*)work_alloc(c, (size_t)nt, &err);
-            if (!err) c->kh_hit = (uint8_t*)work_alloc(c, nb, &err);
-            if (!err) c->kh_cnt = (unsigned*)work_alloc(c, 3 * sizeof(unsigned), &err);
+            if (!err) c->kh_cnt = (unsigned*)work_alloc(c, 4 * sizeof(unsigned), &err);
         }
         if (err) {
             dba_destroy(c);
@@ -1565,7 +1563,11 @@ int dba_restore(dba_ctx* c, const char* path)
     // a file may have been written without the rings of the blocks that fell asleep in its last step
     // (checkpoints flush them now); with the same constants, computing them again is exact
     const dba_config &a = cfg, &b = c->cfg;
-    return reset_work(c, a.dt == b.dt && a.cfl == b.cfl && a.dx == b.dx && a.dy == b.dy && a.kh_gamma == b.kh_gamma);
+    if (a.dt == b.dt && a.cfl == b.cfl && a.dx == b.dx && a.dy == b.dy && a.kh_gamma == b.kh_gamma) {
+        const int st = flush_rings(c);
+        if (st) return st;
+    }
+    return reset_work(c);
 }
 
 int dba_tip_profile(dba_ctx* c, int field, int dz, int* tip_x, int* tip_x_max)

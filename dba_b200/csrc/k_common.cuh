@@ -80,6 +80,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+// A kernel launched with programmatic stream serialization starts when every CTA of the kernel
+// before it has called grid_release or ended; grid_wait waits for that kernel to complete with its
+// writes (every path through such a kernel calls it: what follows waits for this kernel alone)
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // periodic wrap of an index at most one period outside [0, n)
 __device__ __forceinline__ int wrap_p(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 

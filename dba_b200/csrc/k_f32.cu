@@ -17,11 +17,11 @@ cudaError_t launch_gather_lazy(cudaStream_t st, const GridP& g, int B, const flo
     return cudaGetLastError();
 }
 
-cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P, const KHStripP& X)
+cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P)
 {
     const int grid = (g.nb + 255) / 256;
-    if (B == 8) kh_strip_flush<8><<<grid, 256, 0, st>>>(g, f, P, X);
-    else kh_strip_flush<16><<<grid, 256, 0, st>>>(g, f, P, X);
+    if (B == 8) kh_strip_flush<8><<<grid, 256, 0, st>>>(g, f, P);
+    else kh_strip_flush<16><<<grid, 256, 0, st>>>(g, f, P);
     return cudaGetLastError();
 }
 

@@ -205,12 +205,10 @@ template <typename R, int B>
 static int kh_tile_grid_b(int sms, int ntiles)
 {
     const size_t sm = KHTile<R, B>::smem;
-    if constexpr (sizeof(R) == 4)
-        cudaFuncSetAttribute(kh_tile_step<R, B, true, KHStripP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(kh_tile_step<R, B, true, KHNoStrips>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(kh_tile_step<R, B, false, KHNoStrips>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kh_tile_step<R, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kh_tile_step<R, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kh_tile_step<R, B, true, KHNoStrips>, KHTile<R, B>::NT, sm) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kh_tile_step<R, B, true>, KHTile<R, B>::NT, sm) != cudaSuccess ||
         occ < 1)
         occ = 1;
     const int g = occ * sms;
@@ -223,9 +221,27 @@ int kh_tile_grid(int B, int sms, int ntiles)
     return B == 8 ? kh_tile_grid_b<R, 8>(sms, ntiles) : kh_tile_grid_b<R, 16>(sms, ntiles);
 }
 
+// launch that may start before the kernel in front of it in the stream has ended (grid_release there,
+// grid_wait here); captured into a graph as such
+template <typename... K, typename... A>
+static cudaError_t launch_beside(void (*kernel)(K...), int grid, int threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // full tiles by strips; DBA: the others by tiles
 template <int B>
-static cudaError_t kh_strips(bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P,
+static cudaError_t kh_strips(bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P,
                              const KHStripP& X)
 {
     const int sg = (g.nb + 255) / 256;
@@ -234,9 +250,10 @@ static cudaError_t kh_strips(bool dba_mode, int grid, cudaStream_t st, const Gri
     const int units = ((g.nx + KHStrip::OUT - 1) / KHStrip::OUT) * ((g.ny + H - 1) / H);
     const int ug = (units + KHStrip::NT / 32 - 1) / (KHStrip::NT / 32);
     if (dba_mode) {
-        kh_strip_scan<B, true><<<sg, 256, 0, st>>>(g, f, P, X);
-        kh_strip_step<B, true><<<ug, KHStrip::NT, 0, st>>>(g, f, P, X, K, H);
-        kh_tile_step<float, B, true, KHStripP><<<grid, KHTile<float, B>::NT, KHTile<float, B>::smem, st>>>(g, f, P, X);
+        cudaError_t e = launch_beside(kh_strip_scan<B, true>, sg, 256, 0, st, g, f, P, X);
+        if (e == cudaSuccess) e = launch_beside(kh_strip_step<B, true>, units < sms ? units : sms, KHStrip::NTD, 0, st, g, f, P, X, K, H);
+        if (e != cudaSuccess) return e;
+        return launch_beside(kh_tile_step<float, B, true>, grid, KHTile<float, B>::NT, KHTile<float, B>::smem, st, g, f, P);
     } else {
         kh_strip_scan<B, false><<<sg, 256, 0, st>>>(g, f, P, X);
         kh_strip_step<B, false><<<ug, KHStrip::NT, 0, st>>>(g, f, P, X, K, H);
@@ -246,11 +263,11 @@ static cudaError_t kh_strips(bool dba_mode, int grid, cudaStream_t st, const Gri
 
 template <typename R>
 cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
-                           const KHTileP<R>& P, const KHStripP* X)
+                           const KHTileP<R>& P, const KHStripP* X, int sms)
 {
     if (!f.tlist || !f.tctr) return cudaErrorInvalidValue;
     if constexpr (sizeof(R) == 4)
-        if (X) return B == 8 ? kh_strips<8>(dba_mode, grid, st, g, f, P, *X) : kh_strips<16>(dba_mode, grid, st, g, f, P, *X);
+        if (X) return B == 8 ? kh_strips<8>(dba_mode, grid, sms, st, g, f, P, *X) : kh_strips<16>(dba_mode, grid, sms, st, g, f, P, *X);
     // the scan lists the step's tiles (one thread per block), the tile kernel takes them
     const int sg = (int)(((long long)g.nb + 255) / 256 < 65535 ? ((long long)g.nb + 255) / 256 : 65535);
 #define XT(b)                                                                                          \
@@ -258,10 +275,10 @@ cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, cons
         const size_t sm = KHTile<R, b>::smem;                                                          \
         if (dba_mode) {                                                                                \
             kh_tile_scan<R, b, true><<<sg, 256, 0, st>>>(g, f, P);                                     \
-            kh_tile_step<R, b, true, KHNoStrips><<<grid, KHTile<R, b>::NT, sm, st>>>(g, f, P, KHNoStrips{});                     \
+            kh_tile_step<R, b, true><<<grid, KHTile<R, b>::NT, sm, st>>>(g, f, P);                     \
         } else {                                                                                       \
             kh_tile_scan<R, b, false><<<sg, 256, 0, st>>>(g, f, P);                                    \
-            kh_tile_step<R, b, false, KHNoStrips><<<grid, KHTile<R, b>::NT, sm, st>>>(g, f, P, KHNoStrips{});                    \
+            kh_tile_step<R, b, false><<<grid, KHTile<R, b>::NT, sm, st>>>(g, f, P);                    \
         }                                                                                              \
         return cudaGetLastError();                                                                     \
     }
@@ -455,7 +472,7 @@ template cudaError_t launch_kh<REAL_T>(int, bool, int, cudaStream_t, const GridP
 template cudaError_t launch_correct<REAL_T>(int, cudaStream_t, const GridP&, const CorrP<REAL_T>&);
 template int kh_tile_grid<REAL_T>(int, int, int);
 template cudaError_t launch_kh_tile<REAL_T>(int, bool, int, cudaStream_t, const GridP&, const FlagP&, const KHTileP<REAL_T>&,
-                                                    const KHStripP*);
+                                                    const KHStripP*, int);
 template cudaError_t launch_gather<REAL_T>(cudaStream_t, const GridP&, int, int, const REAL_T*, const REAL_T*,
                                            const uint8_t*, size_t, size_t, size_t, double*);
 template cudaError_t launch_kh_prim_blocks<REAL_T>(cudaStream_t, const GridP&, int, const KHP<REAL_T>&, const uint8_t*);

@@ -12,10 +12,9 @@
 //   kh_strip_scan    the bookkeeping of kh_tile_scan, and per tile: full, or listed; persists
 //                    what the neighbours of a block that fell asleep since the step before can read
 //                    stale, computed again from the buffers that step read
-//   kh_strip_step    full tiles; per block: the largest signal speed (CFL) and whether a cell
-//                    passes the wake-up test (a byte per block)
-//   kh_tile_step     (DBA) the listed tiles; then next flags and wake-up scatter of the blocks of
-//                    full tiles
+//   kh_strip_step    full tiles; per block: the largest signal speed (CFL), the wake-up test with its
+//                    scatter
+//   kh_tile_step     (DBA) the listed tiles, beside the strips (grid_release)
 //
 // What bounds it: latency at four warps per scheduler (128 registers), then instruction issue.
 // The tile kernel spends 686 warp instructions on 32 cells: it computes primitives on 400,
@@ -23,7 +22,11 @@
 // shared memory (71 % of that pipe's peak).  One column per lane took 368 instructions on
 // 28 cells and 75 us per regular 2048^2 step, this form 472 on 60 cells and 66.
 // Measured per step, every block active, tile kernel -> this: 2048^2 DBA with the CFL step 120 ->
-// 79 us, regular 115 -> 66; 4096^2 DBA 449 -> 256; 1024^2 DBA 39.5 -> 33.9, regular 36.1 -> 24.
+// 69 us, regular 114 -> 66; 4096^2 DBA 449 -> 246; 1024^2 DBA 36.9 -> 30.7, regular 35.5 -> 23.4.
+// A DBA step's three kernels are launched beside one another (grid_release, grid_wait): the scan
+// starts while the last tiles of the step before end, the strips' CTAs while it runs, and the
+// tiles take the places that strips leave.  In plain order a step that uses no strips took 2 to 5 us
+// more than tiles alone; now -0.7 to +0.9.
 #pragma once
 
 #include "k_common.cuh"
@@ -35,26 +38,37 @@ namespace dba {
 
 struct KHStrip {
     static constexpr int OUT = 60;                       // columns a warp advances: two per lane, lanes 1 .. 30
-    static constexpr int NT = 128;                       // independent warps
-    // Rows a warp walks (a multiple of 16): 32, or 16 where 32 would leave fewer warps than are
-    // resident (148 x 16).  us per regular step: 2048^2 66 / 69, 1024^2 47 / 35.
+    // independent warps, 16 per SM at 128 registers; DBA steps in one CTA per SM
+    static constexpr int NT = 128, NTD = 512;
+    // Rows a warp walks (a multiple of 16): 32, or 16 where 32 would leave most of the 148 x 16
+    // resident warps idle.  us per regular step, 32 / 16 rows: 2048^2 (2240 warps at 32) 66 / 69,
+    // 1024^2 (576) 47 / 35.
     static int rows(int nx, int ny) { return (long long)((nx + OUT - 1) / OUT) * (ny / 32) >= 2000 ? 32 : 16; }
 };
 
-// Whether this step uses the strips: by the full tiles of the step before (either way the
-// results are the same, bit for bit).  A warp walks its unit when any tile of it is full, so
-// the strips' time hardly falls with the number of full tiles, while the tiles that are not
-// full come on top.  2048^2, us per step, tiles alone / with strips: every block active
-// 120 / 79, 97 % 120 / 100, 90 % 116 / 107, 81 % 106 / 110, 63 % 86 / 111; 1024^2: every
-// block 39.5 / 33, 97 % 37.6 / 48.5.  Unused, their two launches and the scan's look at the
-// neighbours cost 5 us.
-// (cnt: X.cnt_prev; before kh_strip_step clears it, X.cnt_next still holds the count that the
-// step before decided by.  After a load cnt_prev is all ones (strips on) and the others are zero: the
-// state's rings are complete.)
+// full[tile]: every block of the 16^2 tile and around it is active in the step last scanned, which took
+// the tile by strips.  Counts of such tiles (whatever took them): of the step before, of this one,
+// and the word that the next step counts into.
+struct KHStripP {
+    uint8_t* full = nullptr;
+    const unsigned* cnt_prev = nullptr;
+    unsigned *cnt_cur = nullptr, *cnt_next = nullptr;
+    unsigned* taken = nullptr;                           // units taken beyond every warp's first
+};
+
+// Whether this step uses the strips: by the full tiles of the step before (either way the results
+// are the same, bit for bit).  A warp walks its unit when any tile of it is full, so scattered
+// quiet spots leave the strips' time as it is, while the tiles that are not full come on top.
+// us per step, tiles / strips, at shares of full tiles (a quiet band; 4 quiet spots; 64):
+//   1024^2 (4096 tiles)  92 % 36.8 / 35.6; 90 % 36.3 / 36.3; 86 % 36.1 / 37.1; 83 % 34.5 / 35.5; 76 % 33.9 / 37.2
+//   1536^2               92 % 69.6 / 46.0; 72 % 57.1 / 39.0; 66 % 56.9 / 47.8; 64 % 71 / 60
+//   2048^2 (16384 tiles) 92 % 114 / 74; 74 % 98.9 / 76.2; 64 % 89 / 75; 60 % 103 / 98; 55 % 79.6 / 74.3;
+//                        45 % 69.7 / 71.5
+// (A restored state starts with a count of all ones: strips on.)
 __device__ __forceinline__ bool kh_strips_on(const GridP& g, const unsigned* cnt)
 {
     const unsigned n = (unsigned)((g.nx / 16) * (g.ny / 16)), lacking = n - min(*cnt, n);
-    return lacking <= (n >= 8192u ? n / 4u : n / 32u);   // 8192 tiles: 2^21 cells
+    return lacking <= (n >= 8192u ? 2u * n / 5u : n / 10u);   // 8192 tiles: 2^21 cells
 }
 
 // one cell's four quantities, and the formulas on them (the blocks that may fall asleep)
@@ -133,7 +147,9 @@ __device__ __forceinline__ bool kh_around(const GridP& g, const uint8_t* w, int 
 {
     const int xm = (bx == 0 ? g.nbx : bx) - 1, xp = bx + 1 == g.nbx ? 0 : bx + 1;
     const int ym = ((by == 0 ? g.nby : by) - 1) * g.nbx, yp = (by + 1 == g.nby ? 0 : by + 1) * g.nbx, yc = by * g.nbx;
-    return w[xm + ym] && w[bx + ym] && w[xp + ym] && w[xm + yc] && w[xp + yc] && w[xm + yp] && w[bx + yp] && w[xp + yp];
+    // (eight loads in flight, not one after the other)
+    const uint8_t a = w[xm + ym], b = w[bx + ym], c = w[xp + ym], d = w[xm + yc], e = w[xp + yc], h = w[xm + yp], i = w[bx + yp], k = w[xp + yp];
+    return (a != 0) & (b != 0) & (c != 0) & (d != 0) & (e != 0) & (h != 0) & (i != 0) & (k != 0);
 }
 
 // Ring persistence of `cnt` blocks that fell asleep, by the warps of a CTA of 256, half a ring each: what
@@ -175,14 +191,6 @@ __device__ __forceinline__ void kh_persist_rings(const GridP& g, const FlagP& f,
     }
 }
 
-// Whether block (bx, by), asleep in this step, has a ring to persist: it fell asleep since the step
-// before, which advanced it by strips.  (A block with an inactive neighbour then was in a listed tile,
-// whose update has persisted it; wake_clr holds the flags of that step until kh_tile_step clears it.)
-__device__ __forceinline__ bool kh_ring_pending(const GridP& g, const FlagP& f, const KHStripP& X, int b, int bx, int by)
-{
-    return f.wake_clr[b] && kh_strips_on(g, X.cnt_next) && kh_around(g, f.wake_clr, bx, by);
-}
-
 template <int B, bool DBA>
 __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
 {
@@ -195,24 +203,37 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
     const int bx = tbx * TB + kq % TB, by = tby * TB + kq / TB, b = bx + g.nbx * by;
     const bool cfl = P.cfl > 0.0;
     __shared__ int s_blk[256], s_cnt;                    // blocks that fell asleep since the step before
+    __shared__ unsigned s_nw;                            // full tiles
     if (DBA) {
-        if (threadIdx.x == 0) s_cnt = 0;
+        grid_release();                                  // kh_strip_step may start, and wait
+        grid_wait();                                     // the step before
+        if (threadIdx.x == 0) {
+            s_cnt = 0;
+            s_nw = 0u;
+        }
         __syncthreads();
     }
     int act = 0, pp = 0;
     bool around = true;                                  // the blocks around this one are active
+    bool on = true;
+    unsigned vm = 0u;
     if (valid) {
+        // (every load that a thread may need in flight at once)
         pp = f.par_cur[b];
         act = DBA ? (f.wake_cur[b] ? 1 : 0) : 1;
-        f.par_nxt[b] = (uint8_t)(pp ^ act);
         if (DBA) {
+            const uint8_t was = X.full[tile];
+            on = kh_strips_on(g, X.cnt_prev);
             around = kh_around(g, f.wake_cur, bx, by);
-            if (!act && kh_ring_pending(g, f, X, b, bx, by)) s_blk[atomicAdd(&s_cnt, 1)] = b;
+            // fell asleep after a step that took its tile by strips
+            if (!act && was) s_blk[atomicAdd(&s_cnt, 1)] = b;
         } else {
-            f.wake_clr[b] = 0;
             f.wake_nxt[b] = 1;
         }
+        f.par_nxt[b] = (uint8_t)(pp ^ act);
+        f.wake_clr[b] = 0;
     }
+    __syncwarp();                                        // the tile's lanes have read its entry
     count_stats(f.stats, act, valid);
     const unsigned ma = __ballot_sync(0xffffffffu, valid && act);
     const unsigned mr = __ballot_sync(0xffffffffu, valid && act && around);
@@ -220,12 +241,19 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
     const int g0 = (threadIdx.x & 31) & ~(NBT - 1);
     constexpr unsigned gm = (1u << NBT) - 1u;
     const unsigned abits = (ma >> g0) & gm, pbits = (mp >> g0) & gm;
-    const bool whole = ((mr >> g0) & gm) == gm, full = whole && (!DBA || kh_strips_on(g, X.cnt_prev));
-    const unsigned nw = __popc(__ballot_sync(0xffffffffu, valid && kq == 0 && whole));
-    if ((threadIdx.x & 31) == 0 && nw) atomicAdd(X.cnt_cur, nw);
-    unsigned vm = 0u;
+    const bool whole = ((mr >> g0) & gm) == gm, full = whole && on;
+    if (DBA) {
+        const unsigned nw = __popc(__ballot_sync(0xffffffffu, valid && kq == 0 && whole));
+        if ((threadIdx.x & 31) == 0 && nw) atomicAdd(&s_nw, nw);
+    }
+    if (it == 0) {
+        *X.cnt_next = 0u;
+        *X.taken = 0u;
+        if (!DBA) *X.cnt_cur = (unsigned)ntiles;
+    }
     if (valid) {
         if (kq == 0) X.full[tile] = full;
+        if (DBA && full) f.next[b] = 0;                  // (kh_strip_step sets it)
         if (cfl) {
             if (full) P.vmax[b] = 0.f;                   // kh_strip_step takes the maximum into it
             else if (!act) vm = __float_as_uint(P.vmax[b]);
@@ -241,19 +269,21 @@ __global__ void __launch_bounds__(256) kh_strip_scan(GridP g, FlagP f, KHTileP<f
         if ((threadIdx.x & 31) == 0 && vm) atomicMax(P.gmax_cur, vm);
     }
     __syncthreads();
+    if (threadIdx.x == 0 && s_nw) atomicAdd(X.cnt_cur, s_nw);
     if (s_cnt) kh_persist_rings(g, f, P, B, s_blk, s_cnt);
 }
 
 // The rings that the next step's scan would persist, ahead of a save: a saved state holds them, since
-// another context that loads it may take its steps with other constants.
+// another context that loads it may take its steps with other constants.  By the flags of the step
+// before: a ring that the tile kernel has persisted is the same computed again.
 template <int B>
-__global__ void __launch_bounds__(256) kh_strip_flush(GridP g, FlagP f, KHTileP<float> P, KHStripP X)
+__global__ void __launch_bounds__(256) kh_strip_flush(GridP g, FlagP f, KHTileP<float> P)
 {
     __shared__ int s_blk[256], s_cnt;
     const int b = blockIdx.x * 256 + threadIdx.x;
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
-    if (b < g.nb && !f.wake_cur[b] && kh_ring_pending(g, f, X, b, b % g.nbx, b / g.nbx)) s_blk[atomicAdd(&s_cnt, 1)] = b;
+    if (b < g.nb && !f.wake_cur[b] && f.wake_clr[b] && kh_around(g, f.wake_clr, b % g.nbx, b / g.nbx)) s_blk[atomicAdd(&s_cnt, 1)] = b;
     __syncthreads();
     if (s_cnt) kh_persist_rings(g, f, P, B, s_blk, s_cnt);
 }
@@ -342,15 +372,18 @@ __device__ __forceinline__ void kh_pair_flux(const KHPairK& K, const Pair4& L, c
 }
 
 template <int B, bool DBA>
-__global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f, KHTileP<float> P, KHStripP X, KHPairK K, int H)
+__global__ void __launch_bounds__(DBA ? KHStrip::NTD : KHStrip::NT, DBA ? 1 : 4) kh_strip_step(GridP g, FlagP f, KHTileP<float> P, KHStripP X, KHPairK K, int H)
 {
-    constexpr int OUT = KHStrip::OUT;
-    if (DBA && blockIdx.x > 0 && !kh_strips_on(g, X.cnt_prev)) return;
+    constexpr int OUT = KHStrip::OUT, NT = DBA ? KHStrip::NTD : KHStrip::NT;
+    if (DBA) {
+        grid_wait();                                     // the scan
+        grid_release();                                  // kh_tile_step works on other tiles
+        if (!kh_strips_on(g, X.cnt_prev)) return;
+    }
     const int lane = threadIdx.x & 31;
     const int nsx = (g.nx + OUT - 1) / OUT;
-    const int u = blockIdx.x * (KHStrip::NT / 32) + (threadIdx.x >> 5);
-    const int sy = u / nsx, sx = u - sy * nsx;
-    const int y0 = sy * H, rows = min(H, g.ny - y0);
+    // (DBA: consecutive units on different SMs)
+    int u = DBA ? (int)(blockIdx.x + gridDim.x * (threadIdx.x >> 5)) : (int)(blockIdx.x * (NT / 32) + (threadIdx.x >> 5));
     const bool cfl = P.cfl > 0.0;
     f2 mh, dtdx;
     {
@@ -358,125 +391,144 @@ __global__ void __launch_bounds__(KHStrip::NT, 4) kh_strip_step(GridP g, FlagP f
         const KHK<float> Kd = kh_strip_consts(P, P.gmax_prev, dt);
         mh = f2_pack(-Kd.hdt, -Kd.hdt);
         dtdx = f2_pack(Kd.dtdx, Kd.dtdx);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *X.cnt_next = 0u;
-            if (cfl) {
-                *P.gmax_clear = 0u;
-                *P.time += dt;
-            }
+        if (!DBA && cfl && blockIdx.x == 0 && threadIdx.x == 0) {   // (DBA: kh_tile_step)
+            *P.gmax_clear = 0u;
+            *P.time += dt;
         }
     }
-    if (y0 >= g.ny || (DBA && !kh_strips_on(g, X.cnt_prev))) return;
-    const int xr = sx * OUT + 2 * lane - 2;              // the lane's first column; past the grid's last one it is no output
-    const bool own = lane >= 1 && lane <= 30 && xr < g.nx;
-    int x = wrap_p(xr, g.nx);
-    while (x >= g.nx) x -= g.nx;                         // (a narrow grid wraps more than once)
+    unsigned vwarp = 0u;
+    bool bad = false;
+    // Regular steps: a unit per warp.  DBA: the warps that are resident at once (what a step without strips
+    // pays for) take one unit each, and further ones from a counter.
+    const int warps = gridDim.x * (NT / 32);
+    auto next_unit = [&]() -> int {
+        int n = 0;
+        if (lane == 0) n = warps + (int)atomicAdd(X.taken, 1u);
+        return __shfl_sync(0xffffffffu, n, 0);
+    };
     const float thr = (float)P.thr;
     const int ntx = g.nx / 16;
     const size_t nx = (size_t)g.nx;
-    if (DBA) {                                           // a unit without a full tile has nothing to do
-        bool any = false;
-        for (int y = y0; y < y0 + rows; y += 16) any |= own && X.full[x / 16 + ntx * (y / 16)];
-        if (!__any_sync(0xffffffffu, any)) return;
-    }
+    for (;; u = next_unit()) {
+        const int sy = u / nsx, sx = u - sy * nsx;
+        const int y0 = sy * H, rows = min(H, g.ny - y0);
+        if (y0 >= g.ny) break;
+        const int xr = sx * OUT + 2 * lane - 2;              // the lane's first column; past the grid's last one it is no output
+        const bool own = lane >= 1 && lane <= 30 && xr < g.nx;
+        int x = wrap_p(xr, g.nx);
+        while (x >= g.nx) x -= g.nx;                         // (a narrow grid wraps more than once)
+        if (DBA) {                                           // a unit without a full tile has nothing to do
+            bool any = false;
+            for (int y = y0; y < y0 + rows; y += 16) any |= own && X.full[x / 16 + ntx * (y / 16)];
+            if (!__any_sync(0xffffffffu, any)) continue;
+        }
 
-    int par = 0;                                         // buffer of the block of the row last loaded
-    auto load = [&](int y) -> Pair4 {                    // conserved fields of row y (wrapped), the block's current buffer
-        const int yw = wrap_p(y, g.ny);
-        if (yw % B == 0 || y < y0 - 1) par = f.par_cur[x / B + g.nbx * (yw / B)] ? 1 : 0;
-        const size_t gi = (size_t)x + nx * yw;
-        Pair4 q;
-        q.a = *reinterpret_cast<const f2*>(P.U[0][par] + gi);
-        q.b = *reinterpret_cast<const f2*>(P.U[1][par] + gi);
-        q.c = *reinterpret_cast<const f2*>(P.U[2][par] + gi);
-        q.d = *reinterpret_cast<const f2*>(P.U[3][par] + gi);
-        return q;
-    };
-    Pair4 up = load(y0 - 2);
-    Pair4 wm = kh_pair_prim(K, up);
-    up = load(y0 - 1);
-    Pair4 wc = kh_pair_prim(K, up);
-    up = load(y0);                                       // conserved fields of row y + 1
-    Pair4 rm = {}, fd = {}, dfx = {};                    // row y - 1: state at its upper face, flux below it, its x flux difference
-    bool hit = false, bad = false;
-    unsigned vblk = 0u, vwarp = 0u;
-    bool on = false;                                     // the row being updated: the lane's cells are of a full tile,
-    int dst = 0;                                         //   and the buffer they go to
+        int par = 0;                                         // buffer of the block of the row last loaded
+        auto load = [&](int y) -> Pair4 {                    // conserved fields of row y (wrapped), the block's current buffer
+            const int yw = wrap_p(y, g.ny);
+            if (yw % B == 0 || y < y0 - 1) par = f.par_cur[x / B + g.nbx * (yw / B)] ? 1 : 0;
+            const size_t gi = (size_t)x + nx * yw;
+            Pair4 q;
+            q.a = *reinterpret_cast<const f2*>(P.U[0][par] + gi);
+            q.b = *reinterpret_cast<const f2*>(P.U[1][par] + gi);
+            q.c = *reinterpret_cast<const f2*>(P.U[2][par] + gi);
+            q.d = *reinterpret_cast<const f2*>(P.U[3][par] + gi);
+            return q;
+        };
+        Pair4 up = load(y0 - 2);
+        Pair4 wm = kh_pair_prim(K, up);
+        up = load(y0 - 1);
+        Pair4 wc = kh_pair_prim(K, up);
+        up = load(y0);                                       // conserved fields of row y + 1
+        Pair4 rm = {}, fd = {}, dfx = {};                    // row y - 1: state at its upper face, flux below it, its x flux difference
+        bool hit = false;
+        unsigned vblk = 0u;
+        bool on = false;                                     // the row being updated: the lane's cells are of a full tile,
+        int dst = 0;                                         //   and the buffer they go to
 #pragma unroll 1
-    for (int y = y0 - 1; y <= y0 + rows; ++y) {
-        Pair4 un = up;
-        if (y < y0 + rows) un = load(y + 2);             // a row ahead of its use
-        Pair4 old = up;                                  // conserved fields of row y - 1, again (L1 holds the last rows)
-        if (y > y0) {
-            const size_t gi = (size_t)x + nx * (y - 1);
-            if ((y - 1) % B == 0) dst = f.par_cur[x / B + g.nbx * ((y - 1) / B)] ? 0 : 1;
-            old.a = *reinterpret_cast<const f2*>(P.U[0][dst ^ 1] + gi);
-            old.b = *reinterpret_cast<const f2*>(P.U[1][dst ^ 1] + gi);
-            old.c = *reinterpret_cast<const f2*>(P.U[2][dst ^ 1] + gi);
-            old.d = *reinterpret_cast<const f2*>(P.U[3][dst ^ 1] + gi);
-        }
-        const Pair4 wp = kh_pair_prim(K, up);
-        const Pair4 gx = kh_pair_grad(K, right4(wc), left4(wc), K.hx), gy = kh_pair_grad(K, wp, wm, K.hy);
-        const Pair4 pc = kh_pair_prime(K, mh, wc, gx, gy);
-        if (y >= y0) {
-            Pair4 fu;                                    // the face below row y
-            {
-                const Pair4 L{fma2(gy.a, K.mey, pc.a), fma2(gy.b, K.mey, pc.b), fma2(gy.d, K.mey, pc.d), fma2(gy.c, K.mey, pc.c)};
-                kh_pair_flux(K, L, rm, fu.a, fu.b, fu.d, fu.c);
-            }
+        for (int y = y0 - 1; y <= y0 + rows; ++y) {
+            Pair4 un = up;
+            if (y < y0 + rows) un = load(y + 2);             // a row ahead of its use
+            Pair4 old = up;                                  // conserved fields of row y - 1, again (L1 holds the last rows)
             if (y > y0) {
-                // update of row y - 1
-                const int yr = y - 1;
-                const int b = x / B + g.nbx * (yr / B);
-                if (yr % B == 0) on = own && (!DBA || X.full[x / 16 + ntx * (yr / 16)]);
-                if (on) {
-                    const size_t gi = (size_t)x + nx * yr;
-                    auto upd = [&](int q, f2 o, f2 d, f2 a, f2 c) -> f2 {   // field q: old value, x flux difference, fluxes above and below
-                        const f2 n = add2(o, mul2(dtdx, add2(sub2(d, a), c), K.nz));
-                        *reinterpret_cast<f2*>(P.U[q][dst] + gi) = n;
-                        return n;
-                    };
-                    const Pair4 n{upd(0, old.a, dfx.a, fu.a, fd.a), upd(1, old.b, dfx.c, fu.c, fd.c),
-                                  upd(2, old.c, dfx.d, fu.d, fd.d), upd(3, old.d, dfx.b, fu.b, fd.b)};
-                    // NaN once any stored value is not finite (times a zero from the parameters)
-                    const f2 chk = fma2(n.a, K.nz, fma2(n.b, K.nz, fma2(n.c, K.nz, mul2(n.d, K.nz, K.nz))));
-                    bad |= !(f2_lo(chk) == 0.f && f2_hi(chk) == 0.f);
-                    if (cfl) {
-                        const Pair4 w = kh_pair_prim(K, n);
-                        vblk = max(vblk, max(__float_as_uint(kh_speed<float>(f2_lo(w.a), f2_lo(w.b), f2_lo(w.c), f2_lo(w.d), K.gams)),
-                                             __float_as_uint(kh_speed<float>(f2_hi(w.a), f2_hi(w.b), f2_hi(w.c), f2_hi(w.d), K.gams))));
+                const size_t gi = (size_t)x + nx * (y - 1);
+                if ((y - 1) % B == 0) dst = f.par_cur[x / B + g.nbx * ((y - 1) / B)] ? 0 : 1;
+                old.a = *reinterpret_cast<const f2*>(P.U[0][dst ^ 1] + gi);
+                old.b = *reinterpret_cast<const f2*>(P.U[1][dst ^ 1] + gi);
+                old.c = *reinterpret_cast<const f2*>(P.U[2][dst ^ 1] + gi);
+                old.d = *reinterpret_cast<const f2*>(P.U[3][dst ^ 1] + gi);
+            }
+            const Pair4 wp = kh_pair_prim(K, up);
+            const Pair4 gx = kh_pair_grad(K, right4(wc), left4(wc), K.hx), gy = kh_pair_grad(K, wp, wm, K.hy);
+            const Pair4 pc = kh_pair_prime(K, mh, wc, gx, gy);
+            if (y >= y0) {
+                Pair4 fu;                                    // the face below row y
+                {
+                    const Pair4 L{fma2(gy.a, K.mey, pc.a), fma2(gy.b, K.mey, pc.b), fma2(gy.d, K.mey, pc.d), fma2(gy.c, K.mey, pc.c)};
+                    kh_pair_flux(K, L, rm, fu.a, fu.b, fu.d, fu.c);
+                }
+                if (y > y0) {
+                    // update of row y - 1
+                    const int yr = y - 1;
+                    const int b = x / B + g.nbx * (yr / B);
+                    if (yr % B == 0) on = own && (!DBA || X.full[x / 16 + ntx * (yr / 16)]);
+                    if (on) {
+                        const size_t gi = (size_t)x + nx * yr;
+                        auto upd = [&](int q, f2 o, f2 d, f2 a, f2 c) -> f2 {   // field q: old value, x flux difference, fluxes above and below
+                            const f2 n = add2(o, mul2(dtdx, add2(sub2(d, a), c), K.nz));
+                            *reinterpret_cast<f2*>(P.U[q][dst] + gi) = n;
+                            return n;
+                        };
+                        const Pair4 n{upd(0, old.a, dfx.a, fu.a, fd.a), upd(1, old.b, dfx.c, fu.c, fd.c),
+                                      upd(2, old.c, dfx.d, fu.d, fd.d), upd(3, old.d, dfx.b, fu.b, fd.b)};
+                        // NaN once any stored value is not finite (times a zero from the parameters)
+                        const f2 chk = fma2(n.a, K.nz, fma2(n.b, K.nz, fma2(n.c, K.nz, mul2(n.d, K.nz, K.nz))));
+                        bad |= !(f2_lo(chk) == 0.f && f2_hi(chk) == 0.f);
+                        if (cfl) {
+                            const Pair4 w = kh_pair_prim(K, n);
+                            vblk = max(vblk, max(__float_as_uint(kh_speed<float>(f2_lo(w.a), f2_lo(w.b), f2_lo(w.c), f2_lo(w.d), K.gams)),
+                                                 __float_as_uint(kh_speed<float>(f2_hi(w.a), f2_hi(w.b), f2_hi(w.c), f2_hi(w.d), K.gams))));
+                        }
+                    }
+                    if ((yr + 1) % B == 0) {                 // a block row ends: its blocks' speeds and tests
+                        if (cfl) {
+                            const unsigned grp = __match_any_sync(0xffffffffu, on ? b : -1);
+                            const unsigned v = __reduce_max_sync(grp, vblk);
+                            if (on && lane == __ffs(grp) - 1 && v) atomicMax(reinterpret_cast<unsigned*>(P.vmax) + b, v);
+                            vwarp = max(vwarp, vblk);
+                            vblk = 0u;
+                        }
+                        if (DBA) {                           // next flag, wake-up of the block and the 8 around it
+                            if (on && hit) {
+                                const int bx = x / B, by = yr / B;
+                                const int xm = (bx == 0 ? g.nbx : bx) - 1, xp = bx + 1 == g.nbx ? 0 : bx + 1;
+                                const int ym = ((by == 0 ? g.nby : by) - 1) * g.nbx, yp = (by + 1 == g.nby ? 0 : by + 1) * g.nbx, yc = by * g.nbx;
+                                uint8_t* w = f.wake_nxt;
+                                f.next[b] = 1;
+                                w[xm + ym] = w[bx + ym] = w[xp + ym] = w[xm + yc] = w[b] = w[xp + yc] = w[xm + yp] = w[bx + yp] = w[xp + yp] = 1;
+                            }
+                            hit = false;
+                        }
                     }
                 }
-                if ((yr + 1) % B == 0) {                 // a block row ends: its blocks' speeds and tests
-                    if (cfl) {
-                        const unsigned grp = __match_any_sync(0xffffffffu, on ? b : -1);
-                        const unsigned v = __reduce_max_sync(grp, vblk);
-                        if (on && lane == __ffs(grp) - 1 && v) atomicMax(reinterpret_cast<unsigned*>(P.vmax) + b, v);
-                        vwarp = max(vwarp, vblk);
-                        vblk = 0u;
-                    }
-                    if (DBA) {
-                        if (on && hit) X.hit[b] = 1;
-                        hit = false;
-                    }
+                fd = fu;
+                if (DBA)                                     // (row y, recorded when its block row is updated)
+                    hit |= kh_metric8(f2_lo(gx.a), f2_lo(gy.a), f2_lo(gx.b), f2_lo(gy.b), f2_lo(gx.c), f2_lo(gy.c), f2_lo(gx.d), f2_lo(gy.d)) > thr ||
+                           kh_metric8(f2_hi(gx.a), f2_hi(gy.a), f2_hi(gx.b), f2_hi(gy.b), f2_hi(gx.c), f2_hi(gy.c), f2_hi(gx.d), f2_hi(gy.d)) > thr;
+                Pair4 fr;
+                {
+                    const Pair4 m{fma2(gx.a, K.mex, pc.a), fma2(gx.b, K.mex, pc.b), fma2(gx.c, K.mex, pc.c), fma2(gx.d, K.mex, pc.d)};
+                    const Pair4 R{fma2(gx.a, K.ex, pc.a), fma2(gx.b, K.ex, pc.b), fma2(gx.c, K.ex, pc.c), fma2(gx.d, K.ex, pc.d)};
+                    kh_pair_flux(K, right4(m), R, fr.a, fr.b, fr.c, fr.d);
                 }
+                const Pair4 fl = left4(fr);
+                dfx = Pair4{sub2(fl.a, fr.a), sub2(fl.b, fr.b), sub2(fl.c, fr.c), sub2(fl.d, fr.d)};
             }
-            fd = fu;
-            if (DBA)                                     // (row y, recorded when its block row is updated)
-                hit |= kh_metric8(f2_lo(gx.a), f2_lo(gy.a), f2_lo(gx.b), f2_lo(gy.b), f2_lo(gx.c), f2_lo(gy.c), f2_lo(gx.d), f2_lo(gy.d)) > thr ||
-                       kh_metric8(f2_hi(gx.a), f2_hi(gy.a), f2_hi(gx.b), f2_hi(gy.b), f2_hi(gx.c), f2_hi(gy.c), f2_hi(gx.d), f2_hi(gy.d)) > thr;
-            Pair4 fr;
-            {
-                const Pair4 m{fma2(gx.a, K.mex, pc.a), fma2(gx.b, K.mex, pc.b), fma2(gx.c, K.mex, pc.c), fma2(gx.d, K.mex, pc.d)};
-                const Pair4 R{fma2(gx.a, K.ex, pc.a), fma2(gx.b, K.ex, pc.b), fma2(gx.c, K.ex, pc.c), fma2(gx.d, K.ex, pc.d)};
-                kh_pair_flux(K, right4(m), R, fr.a, fr.b, fr.c, fr.d);
-            }
-            const Pair4 fl = left4(fr);
-            dfx = Pair4{sub2(fl.a, fr.a), sub2(fl.b, fr.b), sub2(fl.c, fr.c), sub2(fl.d, fr.d)};
+            wm = wc; wc = wp;
+            up = un;
+            rm = Pair4{fma2(gy.a, K.ey, pc.a), fma2(gy.b, K.ey, pc.b), fma2(gy.d, K.ey, pc.d), fma2(gy.c, K.ey, pc.c)};   // (normal velocity third)
         }
-        wm = wc; wc = wp;
-        up = un;
-        rm = Pair4{fma2(gy.a, K.ey, pc.a), fma2(gy.b, K.ey, pc.b), fma2(gy.d, K.ey, pc.d), fma2(gy.c, K.ey, pc.c)};   // (normal velocity third)
+        if (!DBA) break;
     }
     if (bad) raise_status(f.status, 5);
     if (cfl) {

@@ -74,21 +74,6 @@ struct KHTileP {
     KHK<R> Kc;
 };
 
-// What the strips (k_kh_strip.cuh) share with the tile kernel beside them: full[tile], every block
-// of the 16^2 tile and around it is active this step; hit[block], a cell of a full tile's block
-// passes the wake-up test (zero between steps); full tiles of the step before, of this one, and
-// the word the next step counts into.
-struct KHStripP {
-    static constexpr bool on = true;
-    uint8_t* full = nullptr;
-    uint8_t* hit = nullptr;
-    const unsigned* cnt_prev = nullptr;
-    unsigned *cnt_cur = nullptr, *cnt_next = nullptr;
-};
-struct KHNoStrips {
-    static constexpr bool on = false;
-};
-
 // largest signal speed of a cell: sound speed + flow speed
 template <typename R>
 __device__ __forceinline__ float kh_speed(R r, R p, R u, R v, R gam)
@@ -230,10 +215,8 @@ __global__ void __launch_bounds__(256) kh_tile_scan(GridP g, FlagP f, KHTileP<R>
     }
 }
 
-// X: KHStripP beside strips, KHNoStrips alone (a parameter of the kernel, not a test in it: the extra
-// code costs the plain kernel 2 to 5 % in spilled registers)
-template <typename R, int B, bool DBA, typename X>
-__global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_step(GridP g, FlagP f, KHTileP<R> P, X strips)
+template <typename R, int B, bool DBA>
+__global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_step(GridP g, FlagP f, KHTileP<R> P)
 {
     using S = KHTile<R, B>;
     constexpr int NT = S::NT, T = S::T, TB = S::TB, NBT = S::NBT, RB = S::RB, GT = S::GT;
@@ -263,15 +246,38 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
     __shared__ unsigned s_vcta;                 // this CTA's largest speed over its blocks
     __shared__ R s_hdt, s_dtdx;                 // the step's dt-dependent constants
 
+    if constexpr (sizeof(R) == 4 && DBA) grid_release(); // the next step's scan may take its places (k_kh_strip.cuh)
     const int tid = threadIdx.x;
     const int ntx = g.nx / T, nty = g.ny / T, ntiles = ntx * nty;
     const size_t nx = (size_t)g.nx;
     const bool cfl = P.cfl > 0.0;
+    // The step's listed tiles (kh_tile_scan): CTA c's first is entry c, further ones are taken from
+    // the tile queue by thread GT, two tiles ahead: during phase 2 of tile i (GT has no phase-2 item)
+    // it reads the list entry of tile i + 2, taken during tile i - 1, into slot (i + 2) % 4 and takes
+    // the entry for tile i + 3, so the counter's atomic and the list load are never waited for
+    // on a barrier's path -- nor, at the start, behind the step's dt.
+    const int cnt = (int)min(__ldcg(f.tctr), (unsigned)ntiles);
+    int k_pend = 0;
+    auto take = [&](int k, int slot) {
+        if (k < cnt) {
+            s_tile[slot] = __ldcg(f.tlist + 2 * (size_t)k);
+            s_tmeta[slot] = (unsigned)__ldcg(f.tlist + 2 * (size_t)k + 1);
+        } else {
+            s_tile[slot] = -1;
+        }
+    };
+    if (tid == GT) {
+        k_pend = (int)(gridDim.x + atomicAdd(f.tctr + 1, 2u));
+        const int e = __ldcg(f.tlist + 2 * (size_t)blockIdx.x);   // (the grid has no more CTAs than tiles)
+        const unsigned m = (unsigned)__ldcg(f.tlist + 2 * (size_t)blockIdx.x + 1);
+        s_tile[0] = (int)blockIdx.x < cnt ? e : -1;
+        s_tmeta[0] = m;
+    }
     if (tid == 0) {
         double dt = P.dt;
         if (cfl) {
             dt = P.cfl * P.hmin / (double)__uint_as_float(*P.gmax_prev);
-            if (!X::on && blockIdx.x == 0) {             // (kh_strip_step does it where it runs)
+            if (blockIdx.x == 0) {
                 *P.gmax_clear = 0u;
                 *P.time += dt;
             }
@@ -397,30 +403,9 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
                 for (int q = 0; q < 4; ++q) f.bsum[(size_t)q * g.nb + b] = s_bsum[q][tid];
         }
     };
-    // The step's listed tiles (kh_tile_scan) are taken from the tile queue by thread GT,
-    // two tiles ahead: during phase 2 of tile i (GT has no phase-2 item) it reads the
-    // list entry of tile i + 2, taken during tile i - 1, into slot (i + 2) % 4 and takes
-    // the entry for tile i + 3, so the counter's atomic and the list load are never
-    // waited for on a barrier's path.
-    const int cnt = (int)min(__ldcg(f.tctr), (unsigned)ntiles);
-    int k_pend = 0;
-    auto take = [&](int k, int slot) {
-        if (k < cnt) {
-            s_tile[slot] = __ldcg(f.tlist + 2 * (size_t)k);
-            s_tmeta[slot] = (unsigned)__ldcg(f.tlist + 2 * (size_t)k + 1);
-        } else {
-            s_tile[slot] = -1;
-        }
-    };
-    if (tid == GT) {
-        const int k = (int)atomicAdd(f.tctr + 1, 2u);
-        take(k, 0);
-        take(k + 1, 1);
-        k_pend = (int)atomicAdd(f.tctr + 1, 1u);
-    }
-    __syncthreads();
     if (s_tile[0] >= 0) {
         neighbourhood(s_tile[0], 0);
+        if (tid == GT) take(k_pend++, 1);
         __syncthreads();
         prefetch(tile_at(s_tile[0]), 0);
         cp_async_wait0();
@@ -488,7 +473,7 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
             }
         } else if (tid == GT) {
             take(k_pend, (i + 2) & 3);           // slot (i + 2) % 4 held tile i - 2
-            k_pend = (int)atomicAdd(f.tctr + 1, 1u);
+            k_pend = (int)(gridDim.x + atomicAdd(f.tctr + 1, 1u));
         }
         __syncthreads();
 
@@ -649,23 +634,8 @@ __global__ void __launch_bounds__(KHTile<R, B>::NT, KHTile<R, B>::MINB) kh_tile_
     if (i > 0) tile_end(i - 1);
     __syncthreads();
     if (cfl && tid == 0) atomicMax(P.gmax_cur, s_vcta);
-    if constexpr (DBA && X::on) {
-        // the flags of the step before are cleared here, and the blocks of full tiles get their next
-        // flags and wake their neighbours
-        for (int b = blockIdx.x * NT + tid; b < g.nb; b += gridDim.x * NT) {
-            f.wake_clr[b] = 0;
-            const int bx = b % g.nbx, by = b / g.nbx;
-            if (!strips.full[bx / TB + ntx * (by / TB)]) continue;
-            const int h = strips.hit[b];
-            f.next[b] = (uint8_t)h;
-            if (!h) continue;
-            strips.hit[b] = 0;
-            const int xm = (bx == 0 ? g.nbx : bx) - 1, xp = bx + 1 == g.nbx ? 0 : bx + 1;
-            const int ym = ((by == 0 ? g.nby : by) - 1) * g.nbx, yp = (by + 1 == g.nby ? 0 : by + 1) * g.nbx, yc = by * g.nbx;
-            uint8_t* w = f.wake_nxt;
-            w[xm + ym] = w[bx + ym] = w[xp + ym] = w[xm + yc] = w[b] = w[xp + yc] = w[xm + yp] = w[bx + yp] = w[xp + yp] = 1;
-        }
-    }
+    // launched beside kh_strip_step, whose tiles are others; the next step waits for both
+    if constexpr (sizeof(R) == 4 && DBA) grid_wait();
     if (tid == GT) tile_queue_done(f);
 }
 

@@ -85,14 +85,14 @@ inline bool kh_tiles_ok(int D, int B, int nx, int ny)
 }
 // Whether its fully active regions go through strips (k_kh_strip.cuh): FP32, and enough cells for
 // the strips' warps to fill the GPU.  us per step, DBA with every block active, tiles / strips:
-// 512^2 18.6 / 26, 1024^2 39.4 / 35.4, 2048^2 120 / 78.
+// 512^2 18.6 / 26, 1024^2 36.9 / 30.7, 2048^2 120 / 69.
 inline bool kh_strips_ok(int precision_bytes, int nx, int ny) { return precision_bytes == 4 && (long long)nx * ny >= 1 << 20; }
 template <typename R> int kh_tile_grid(int B, int sms, int ntiles);
 template <typename R>
 cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,
-                           const KHTileP<R>& P, const KHStripP* X);   // X: null without strips
-// rings of the blocks that the next step finds asleep (k_kh_strip.cuh); f, P, X: of the next step
-cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P, const KHStripP& X);
+                           const KHTileP<R>& P, const KHStripP* X, int sms);   // X: null without strips
+// rings of the blocks that the next step finds asleep (k_kh_strip.cuh); f, P: of the next step
+cudaError_t launch_kh_strip_flush(int B, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P);
 // out[k] = buf[par[owner(cell)]][start + k*stride] for k < count (par may be null -> buffer 0)
 template <typename R>
 cudaError_t launch_gather(cudaStream_t st, const GridP& g, int B, int D, const R* b0, const R* b1, const uint8_t* par,
