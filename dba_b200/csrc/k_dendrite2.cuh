@@ -12,9 +12,10 @@
 // the parities around it in one round trip and needs three barriers; the owned form needs
 // seven per round, but packs active blocks into rounds and has no idle CTAs, which counts
 // where most tiles sleep and there are more of them than the GPU holds (dendrite2_tiled).
-// us per step, owned / tiles: every block 512^2 FP64 8.2 / 6.3, 1536^2 FP32 4^2 blocks 72 / 29;
-// DBA 512^2 FP32 5.0 / 4.5, 256 x 200 FP64 5.1 / 4.5, 768 x 800 FP32 6.2 / 5.1; 512^2 FP64 5.1 /
-// 5.3, 1024^2 FP64 7.6 / 8.5, 1536^2 9.3 / 13 (with a tile list).
+// us per step, owned / tiles: every block 512^2 FP64 8.2 / 5.9; DBA 512^2 FP32 4.9 / 3.7 (6 % active) and
+// 6.2 / 4.4 (16 %), 416^2 FP64 5.8 / 4.2; 512^2 FP64 5.1 / 5.3, 1024^2 FP64 7.6 / 8.5, 1536^2 9.3 / 13
+// (with a tile list).  Both since a step's CTAs start as the last ones of the step before end:
+// 0.3 to 0.4 us less.
 #pragma once
 
 #include <type_traits>
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(256, Den2<R, B>::MINB) dendrite2_step(GridP g,
     const int tid = threadIdx.x, nb = g.nb, w = tid >> 5, lane = tid & 31;
     const int ntx = (g.nx + S::TX - 1) / S::TX, ty = blockIdx.x / ntx, tx = blockIdx.x - ty * ntx;
     const int X0 = tx * S::TX, Y0 = ty * S::TY;
+    grid_wait();                                         // the step before
     if (tid < S::NBT) {
         s_hit[0][tid] = 0;
         s_hit[1][tid] = 0;
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(kThreads) dendrite2_owned(GridP g, FlagP f, De
     const R dt = (R)P.dt, delta = (R)P.delta, eps2 = (R)P.eps2, gam = (R)P.gamma;
     const R thr_p = (R)P.thr_p, thr_p_hi = (R)P.thr_p_hi, thr_T = (R)P.thr_T;
 
+    grid_wait();                                         // the step before
     for (long long j0 = 0; blockIdx.x + (long long)G * j0 < nb; j0 += NT) {
         const long long bl = blockIdx.x + (long long)G * (j0 + tid);
         const bool valid = bl < nb;

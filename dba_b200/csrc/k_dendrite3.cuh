@@ -20,8 +20,9 @@
 // and dropped: CTAs that stay and take tiles from a counter two ahead, 70.7 against 67.7 us
 // (fewer round trips per tile, but fewer CTAs in flight).
 // Measured per step, before -> now: 256^3 FP64 in 4^3 blocks (16 % p-, 44 % T-active) 214 ->
-// 67.7 us, in 8^3 blocks 116 -> 70.8; 200 x 136 x 104 FP32 in 8^3 blocks, every block,
-// 42.7 -> 25.1, in 4^3 blocks 84.9 -> 28.8.
+// 66.4 us, in 8^3 blocks 116 -> 70; 200 x 136 x 104 FP32 in 8^3 blocks, every block,
+// 42.7 -> 24.6, in 4^3 blocks 84.9 -> 28.5.  A grid that is nearly all asleep was faster one block
+// at a time: 128^3 FP64 0.6 % p-active 7.7 -> 9.9, 4 % 16.5 -> 12.1.
 #pragma once
 
 #include "k_common.cuh"
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(256) dendrite_scan(GridP g, FlagP f, int ntile
     const int it = blockIdx.x * 256 + threadIdx.x;       // the grid covers ntiles * NBT items
     const int tile = it / S::NBT, k = it % S::NBT;
     const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
+    grid_wait();                                         // the step before
     const uint4 m = den_blocks<S, DBA>(g, f, tile < ntiles, tx, ty, tz, k);
     const bool take = k == 0 && (m.x | m.y) != 0;
     const unsigned mt = __ballot_sync(0xffffffffu, take);
@@ -204,6 +206,8 @@ __global__ void __launch_bounds__(256, Den3<R, B>::MINB) dendrite3_step(GridP g,
     __shared__ uint8_t s_order[S::NBT];                  // the tile's active blocks, those active in p first
     const int tid = threadIdx.x, nb = g.nb, w = tid >> 5;
     __shared__ uint4 s_mask;
+    grid_wait();                                         // the scan, or the step before
+    if (LIST) grid_release();
     const int cnt = LIST ? (int)min(__ldcg(f.tctr), (unsigned)ntiles) : ntiles;
     if (LIST && blockIdx.x == 0 && tid == 0)             // the next step's count: the other of the pair
         *reinterpret_cast<unsigned*>(reinterpret_cast<uintptr_t>(f.tctr) ^ sizeof(unsigned)) = 0u;

@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(256) dendrite3_tile_scan(GridP g, FlagP f)
     const int nb = g.nb;
     const int ntx = (g.nx + TX - 1) / TX, nty = g.ny / B, ntz = g.nz / B;
     const long long nitems = (long long)ntx * nty * ntz * TBX;
+    grid_release();
+    grid_wait();
     for (long long t0 = (long long)blockIdx.x * blockDim.x; t0 < nitems; t0 += (long long)gridDim.x * blockDim.x) {
         const long long it = t0 + threadIdx.x;
         const int tile = (int)(it / TBX), kq = (int)(it % TBX);
@@ -235,15 +237,17 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
         }
     };
 
-    // The step's listed tiles (dendrite3_tile_scan) are taken from the tile queue by
-    // thread GT, two tiles ahead: during tile i it reads the list entry of tile i + 2
-    // (taken during tile i - 1) into slot (i + 2) % 4 and takes the entry for tile i + 3,
-    // so neither the counter's atomic nor the list load is waited for on a barrier's
+    // The step's listed tiles (dendrite3_tile_scan): CTA c's first is entry c, further ones are
+    // taken from the tile queue by thread GT, two tiles ahead: during tile i it reads the list entry
+    // of tile i + 2 (taken during tile i - 1) into slot (i + 2) % 4 and takes the entry for tile
+    // i + 3, so neither the counter's atomic nor the list load is waited for on a barrier's
     // path.  Slot (i + 2) % 4 held tile i - 2, whose bookkeeping ended before the
     // barrier that closed tile i - 1's staging; tile i - 1's slot is read by its
     // bookkeeping after the next barrier.  Two barriers per tile: tile i - 1's update
     // has ended at the one that opens tile i, where its bookkeeping runs (wake tests
     // double-buffered by tile parity), and the stage tile i + 1 refills is free there.
+    grid_wait();                                 // the scan
+    grid_release();
     const int cnt = (int)min(__ldcg(f.tctr), (unsigned)(ntx * nty * (g.nz / B)));
     int k_pend = 0;
     auto entry = [&](int k, int slot) {
@@ -255,14 +259,16 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
         }
     };
     if (tid == GT) {
-        const int k = (int)atomicAdd(f.tctr + 1, 2u);
-        entry(k, 0);
-        entry(k + 1, 1);
-        k_pend = (int)atomicAdd(f.tctr + 1, 1u);
+        k_pend = (int)(gridDim.x + atomicAdd(f.tctr + 1, 2u));
+        const int e = __ldcg(f.tlist + 2 * (size_t)blockIdx.x);   // (the grid has no more CTAs than tiles)
+        const unsigned m = (unsigned)__ldcg(f.tlist + 2 * (size_t)blockIdx.x + 1);
+        s_tile[0] = (int)blockIdx.x < cnt ? e : -1;
+        s_tmeta[0] = m;
     }
     __syncthreads();
         if (s_tile[0] >= 0) {
             build_nbr(0, 0);
+            if (tid == GT) entry(k_pend++, 1);
             __syncthreads();
             issue(0, 0);
         }
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
             if (more) build_nbr(ns, st ^ 1);
             if (tid == GT) {
                 entry(k_pend, (i + 2) & 3);
-                k_pend = (int)atomicAdd(f.tctr + 1, 1u);
+                k_pend = (int)(gridDim.x + atomicAdd(f.tctr + 1, 1u));
             }
             __syncthreads();                     // next table ready; stage st^1 free; tile i - 1 done
             if (i > 0) bookkeep(i - 1);

@@ -80,14 +80,9 @@ cudaError_t launch_dendrite3_tiles(bool dba_mode, int grid, cudaStream_t st, con
     if (!f.tlist || !f.tctr) return cudaErrorInvalidValue;
     // the scan lists the step's tiles (one thread per block), the tile kernel takes them
     const int sg = (int)std::min<long long>(((long long)g.nb + 255) / 256, 65535);
-    if (dba_mode) {
-        dendrite3_tile_scan<true><<<sg, 256, 0, st>>>(g, f);
-        dendrite3_tile_step<true><<<grid, DenTile::NT, DenTile::smem, st>>>(g, f, P);
-    } else {
-        dendrite3_tile_scan<false><<<sg, 256, 0, st>>>(g, f);
-        dendrite3_tile_step<false><<<grid, DenTile::NT, DenTile::smem, st>>>(g, f, P);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = launch_beside(dba_mode ? dendrite3_tile_scan<true> : dendrite3_tile_scan<false>, sg, 256, 0, st, g, f);
+    if (e != cudaSuccess) return e;
+    return launch_beside(dba_mode ? dendrite3_tile_step<true> : dendrite3_tile_step<false>, grid, DenTile::NT, DenTile::smem, st, g, f, P);
 }
 
 int modelb_tile_grid(int B, int sms, int ntiles)
@@ -102,14 +97,9 @@ static cudaError_t modelb_tiles(bool dba_mode, bool bulk, int grid, cudaStream_t
     const MBPairP K = make_pair_params(P);
     const size_t sm = MBTile<B>::smem;
     const int nt = MBTile<B>::NT;
-    if (bulk) {
-        if (dba_mode) modelb_tile_step<B, kMBTileRows, true, true, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
-        else modelb_tile_step<B, kMBTileRows, false, true, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
-    } else {
-        if (dba_mode) modelb_tile_step<B, kMBTileRows, true, false, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
-        else modelb_tile_step<B, kMBTileRows, false, false, RAG><<<grid, nt, sm, st>>>(g, f, P, K, Q, L);
-    }
-    return cudaGetLastError();
+    auto kernel = bulk ? (dba_mode ? modelb_tile_step<B, kMBTileRows, true, true, RAG> : modelb_tile_step<B, kMBTileRows, false, true, RAG>)
+                       : (dba_mode ? modelb_tile_step<B, kMBTileRows, true, false, RAG> : modelb_tile_step<B, kMBTileRows, false, false, RAG>);
+    return launch_beside(kernel, grid, nt, sm, st, g, f, P, K, Q, L);
 }
 
 cudaError_t launch_modelb_tiles(int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,

@@ -10,8 +10,7 @@ cudaError_t launch_reduce(cudaStream_t st, const double* bsum, int nb, int nq, d
                           double* avg, double ncells)
 {
     int J = (nb + 1023) / 1024;
-    cons_reduce<<<J, 1024, 0, st>>>(bsum, nb, nq, l1, J, ticket, avg, ncells);
-    return cudaGetLastError();
+    return launch_beside(cons_reduce, J, 1024, 0, st, bsum, nb, nq, l1, J, ticket, avg, ncells);
 }
 
 }  // namespace dba

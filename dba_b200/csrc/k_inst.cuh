@@ -13,6 +13,28 @@ static int grid_of(const void* kern, size_t smem, int sms)
     return occ * sms;
 }
 
+// Launch that may start before the kernel in front of it in the stream has ended (grid_release there,
+// grid_wait here); captured into a graph as such.  A kernel that does not release lets the next
+// one in as its last CTAs end: us per step, plain / so: 512^2 FP64 dendrite 5.06 / 4.66, 256 x 200
+// FP64 Model B (two kernels) 7.7 / 7.05, 768^2 conserved (four) 48.8 / 47.9, 2048^2 FP32 39.1 / 39.0.
+// An early release only where the next kernel's CTAs are few or take tiles from a counter: others
+// crowd on the SMs that are free first (160^3 FP64 dendrite 13.8 / 15.0).
+template <typename... K, typename... A>
+static cudaError_t launch_beside(void (*kernel)(K...), int grid, int threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 #define DBA_DEN_SHAPES(X) X(2, 4) X(2, 8) X(2, 16) X(2, 32) X(3, 4) X(3, 8)
 #define DBA_MB_SHAPES(X) X(2, 4) X(2, 8) X(2, 16) X(2, 32) X(3, 4) X(3, 8)
 #define DBA_KH_SHAPES(X) X(4) X(8) X(16)
@@ -63,33 +85,24 @@ static cudaError_t den3_launch(bool dba_mode, int grid, cudaStream_t st, const G
     using S = Den3<R, B>;
     const int nt = dendrite3_tiles(g.nx, g.ny, g.nz);
     if (!dendrite3_listed(nt, grid)) {
-        if (dba_mode) dendrite3_step<R, B, true, false><<<nt, S::NT, S::smem, st>>>(g, f, P, nt);
-        else dendrite3_step<R, B, false, false><<<nt, S::NT, S::smem, st>>>(g, f, P, nt);
-        return cudaGetLastError();
+        return launch_beside(dba_mode ? dendrite3_step<R, B, true, false> : dendrite3_step<R, B, false, false>, nt, S::NT, S::smem, st, g, f, P, nt);
     }
     // 8 times as many CTAs as are resident: fewer listed tiles than that (most DBA steps) get
     // one CTA each, and an unused CTA ends after reading the count
     if (!f.tlist || !f.tctr) return cudaErrorInvalidValue;
     const int ng = 8 * grid < nt ? 8 * grid : nt;
     const int sg = (int)(((long long)nt * S::NBT + 255) / 256);
-    if (dba_mode) {
-        dendrite_scan<S, true><<<sg, 256, 0, st>>>(g, f, nt);
-        dendrite3_step<R, B, true, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
-    } else {
-        dendrite_scan<S, false><<<sg, 256, 0, st>>>(g, f, nt);
-        dendrite3_step<R, B, false, true><<<ng, S::NT, S::smem, st>>>(g, f, P, nt);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = launch_beside(dba_mode ? dendrite_scan<S, true> : dendrite_scan<S, false>, sg, 256, 0, st, g, f, nt);
+    if (e != cudaSuccess) return e;
+    return launch_beside(dba_mode ? dendrite3_step<R, B, true, true> : dendrite3_step<R, B, false, true>, ng, S::NT, S::smem, st, g, f, P, nt);
 }
 
 template <typename R, int B>
 static cudaError_t den2_launch(bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f, const DenP<R>& P)
 {
     const int nt = dendrite2_tiles(B, g.nx, g.ny);
-    if (!dendrite2_tiled(sizeof(R), dba_mode, nt, sms)) dendrite2_owned<R, B><<<grid, kThreads, 0, st>>>(g, f, P);
-    else if (dba_mode) dendrite2_step<R, B, true><<<nt, kThreads, 0, st>>>(g, f, P);
-    else dendrite2_step<R, B, false><<<nt, kThreads, 0, st>>>(g, f, P);
-    return cudaGetLastError();
+    if (!dendrite2_tiled(sizeof(R), dba_mode, nt, sms)) return launch_beside(dendrite2_owned<R, B>, grid, kThreads, 0, st, g, f, P);
+    return launch_beside(dba_mode ? dendrite2_step<R, B, true> : dendrite2_step<R, B, false>, nt, kThreads, 0, st, g, f, P);
 }
 
 template <typename R>
@@ -138,14 +151,9 @@ static cudaError_t mb_split(bool dba_mode, cudaStream_t st, const GridP& g, cons
     using S = MBShape<R, D, B>;
     const int nt = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY) * (D == 3 ? (g.nz + S::TZ - 1) / S::TZ : 1);
     const size_t sc = P.conserved ? S::smem_cons : S::smem_mu;
-    if (dba_mode) {
-        modelb_mu<R, D, B, true><<<nt, S::NT, S::smem_mu, st>>>(g, f, P);
-        modelb_update<R, D, B, true><<<nt, S::NT, sc, st>>>(g, f, P);
-    } else {
-        modelb_mu<R, D, B, false><<<nt, S::NT, S::smem_mu, st>>>(g, f, P);
-        modelb_update<R, D, B, false><<<nt, S::NT, sc, st>>>(g, f, P);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = launch_beside(dba_mode ? modelb_mu<R, D, B, true> : modelb_mu<R, D, B, false>, nt, S::NT, S::smem_mu, st, g, f, P);
+    if (e != cudaSuccess) return e;
+    return launch_beside(dba_mode ? modelb_update<R, D, B, true> : modelb_update<R, D, B, false>, nt, S::NT, dba_mode ? sc : S::smem_mu, st, g, f, P);
 }
 
 template <typename R>
@@ -162,9 +170,8 @@ cudaError_t launch_modelb(int D, int B, bool dba_mode, int grid, cudaStream_t st
 #define XF(b)                                                                                   \
     if (B == b) {                                                                               \
         const size_t sm = MBFastShape<b>::smem;                                                 \
-        if (dba_mode) modelb_fast_step<b, true><<<grid, kThreads, sm, st>>>(g, f, FP, FB, L);   \
-        else modelb_fast_step<b, false><<<grid, kThreads, sm, st>>>(g, f, FP, FB, L);           \
-        return cudaGetLastError();                                                              \
+        return launch_beside(dba_mode ? modelb_fast_step<b, true> : modelb_fast_step<b, false>, \
+                             grid, kThreads, sm, st, g, f, FP, FB, L);                          \
     }
             XF(4) XF(8) XF(16) XF(32)
 #undef XF
@@ -221,24 +228,6 @@ int kh_tile_grid(int B, int sms, int ntiles)
     return B == 8 ? kh_tile_grid_b<R, 8>(sms, ntiles) : kh_tile_grid_b<R, 16>(sms, ntiles);
 }
 
-// launch that may start before the kernel in front of it in the stream has ended (grid_release there,
-// grid_wait here); captured into a graph as such
-template <typename... K, typename... A>
-static cudaError_t launch_beside(void (*kernel)(K...), int grid, int threads, size_t smem, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // full tiles by strips; DBA: the others by tiles
 template <int B>
 static cudaError_t kh_strips(bool dba_mode, int grid, int sms, cudaStream_t st, const GridP& g, const FlagP& f, const KHTileP<float>& P,
@@ -290,8 +279,7 @@ cudaError_t launch_kh_tile(int B, bool dba_mode, int grid, cudaStream_t st, cons
 template <typename R>
 cudaError_t launch_correct(int grid, cudaStream_t st, const GridP& g, const CorrP<R>& P)
 {
-    cons_correct<R><<<grid, kThreads, 0, st>>>(g, P);
-    return cudaGetLastError();
+    return launch_beside(cons_correct<R>, grid, kThreads, 0, st, g, P);
 }
 
 template <typename R>

@@ -37,7 +37,11 @@
 // 64 registers leave four CTAs per SM: 3 CTAs at 80 registers took 792 us where 4 take 708.
 // Measured per step, every block active, before -> now: 256^3 FP64 in 4^3 blocks 5167 ->
 // 708 us, 192^3 FP32 in 8^3 blocks (regular) 554 -> 168 us, 4^3 blocks 1088 -> 187 us;
-// 768^2 FP64 in 4^2 blocks 72.9 -> 34.2 us, conserved in 16^2 blocks 69 -> 54 us.
+// 768^2 FP64 in 4^2 blocks 72.9 -> 33.5 us, conserved in 16^2 blocks 67.5 -> 47.9 us.  A 2-D grid of
+// many tiles that is nearly all asleep was faster one block at a time (idle CTAs of two
+// kernels): 1024^2 in 4^2 blocks 2 % active 10.0 -> 16.3, 12 % 20.5 -> 24.0, 43 % 62 -> 36.
+// Several tiles per CTA, their flags read at once, took 13.2 and 20.6 there, but 38.1 at 43 %
+// and two registers more than all other grids have.
 // The Nz == 1 form keeps the reference's 27-term sum with the z neighbours
 // wrapped onto the cell itself.
 #pragma once
@@ -291,6 +295,7 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     const int tid = threadIdx.x;
     const MBTileAt<S, D, B> t(g);
     const int nb = g.nb;
+    grid_wait();                                         // the step before
 
     if (tid < 32) {                                      // bookkeeping: the tile's blocks on one warp
         const int b = tid < S::NBT ? t.block(g, tid) : -1;
@@ -402,6 +407,7 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     __shared__ double s_bsum[3][S::NBT];
     const int tid = threadIdx.x;
     const MBTileAt<S, D, B> t(g);
+    grid_wait();                                         // modelb_mu
     if (tid < 32) {
         const int b = tid < S::NBT ? t.block(g, tid) : -1;
         int act = 0, pp = 0;

@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(kThreads) modelb_fast_step(GridP g, FlagP f, M
     const int tid = threadIdx.x;
     const int G = gridDim.x;
     const int nb = g.nb;
+    grid_wait();                        // the step before
     if (tid < 3) {
         s_Cf[tid] = lazy_offset(L, tid);
         s_fix[tid] = 0ull;

@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(256 / R, 4)
     const int ntx = (g.nx + T - 1) / T, nty = (g.ny + T - 1) / T, ntiles = ntx * nty;
     const size_t nx = (size_t)g.nx;
     const bool ghosts = g.ob0 > 0 || g.ob1 < g.nby;     // a slab with ghost block rows
+    grid_wait();                         // the step before
     if (tid < 3) {
         s_Cf[tid] = lazy_offset(L, tid);
         s_fix[tid] = 0ull;

@@ -52,6 +52,7 @@ static __global__ void __launch_bounds__(1024) cons_reduce(const double* bsum, i
     __shared__ double s32[4][32];
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    grid_wait();                                 // the step's kernels
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     const long long i = (long long)blockIdx.x * 1024 + threadIdx.x;
     for (int q = 0; q < nq; ++q) v[q] = i < nb ? bsum[(size_t)q * nb + i] : 0.0;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(kThreads) cons_correct(GridP g, CorrP<R> P)
     struct alignas(16) Piece { R v[PC]; };
     const int npr = g.nx / PC;                   // pieces per row
     const unsigned np = (unsigned)npr * g.ny * g.nz;
+    grid_wait();                                 // cons_reduce
     double a[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) a[q] = q < P.nq ? P.avg[q] : 0.0;

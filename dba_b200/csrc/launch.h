@@ -40,15 +40,17 @@ int dendrite3_tile_grid(int sms, int ntiles);
 // tiles of the general 3-D dendrite kernel (k_dendrite3.cuh)
 inline int dendrite3_tiles(int nx, int ny, int nz) { return ((nx + 31) / 32) * ((ny + 7) / 8) * ((nz + 7) / 8); }
 // Whether it works from a list (resident: CTAs on the GPU at once).  The scan is a launch of
-// its own, about 3 us; without it each idle tile costs a CTA that reads its flags and ends.
-// us per step, list / none: FP64 4^3 blocks 128^3 (2.3 tiles per resident CTA) 30.4 / 26.9,
-// 192x160x96 (3.2) 26.9 / 25.1, 256^3 (18) 67.7 / 76.7; FP32 8^3 200x136x104 (2.1)
-// 19.5 / 17.0, 256^3 (11) 31.7 / 38.0.
-// FP32 8^3 grids that need a list take the double-buffered tiles of k_dendrite_tile.cuh instead:
-// 512^3 dense 745 against 779 us, 256^3 106 against 107, but 200x136x104 29.6 against 25.1.
+// its own; without it each idle tile costs a CTA that reads its flags and ends.
+// us per step, list / none: FP64 4^3 blocks 128^3 (2.3 tiles per resident CTA) 18.2 / 15.9,
+// 192x160x96 (3.2) 14.4 / 13.8 and 22.3 / 22.0, 256^3 (18) 67.7 / 76.7; FP32 8^3 200x136x104 (2.1)
+// 12.6 / 11.7, 18.5 / 18.5; 256x176x128 (3.8) 20.0 / 22.0.
+// FP32 8^3 grids that need a list take the double-buffered tiles of k_dendrite_tile.cuh instead (us
+// per step against this kernel's list): 512^3 dense 745 / 779; 232^3 21.6 / 23.0 and 48 / 52.
 inline bool dendrite3_listed(int tiles, int resident) { return tiles > 4 * resident; }
-// 2-D: whether a step goes by tiles (k_dendrite2.cuh, with the figures): every regular step; DBA steps
-// while the tiles are about as many as the GPU holds at once (148 x 5 in FP64, 148 x 6 in FP32)
+// 2-D: whether a step goes by tiles (k_dendrite2.cuh): every regular step, and DBA steps up to 5 tiles per
+// SM in FP64, 9 in FP32.  us per step, owned / tiles: FP64 864^2 in 32^2 blocks (729 tiles) 8 % active
+// 8.1 / 6.3, 17 % 8.3 / 8.7; 512^2 in 8^2 blocks (1024) 5.1 / 5.3; FP32 512^2 in 8^2 blocks
+// (1024) 4.9 / 3.7; 1152^2 in 32^2 blocks (1296) 8.3 / 5.0.
 inline int dendrite2_tiles(int B, int nx, int ny) { return ((nx + 31) / 32) * (B > 8 ? ny / B : (ny + 7) / 8); }
 inline bool dendrite2_tiled(int precision_bytes, bool dba_mode, int tiles, int sms)
 {
