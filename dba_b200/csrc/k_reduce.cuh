@@ -67,6 +67,7 @@ static __global__ void __launch_bounds__(1024) cons_reduce(const double* bsum, i
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();                         // the other warps' totals, seen at the barrier, before the ticket
         unsigned prev = atomicAdd(ticket, 1u);
         s_last = (prev == gridDim.x - 1);
     }
