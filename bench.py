@@ -236,9 +236,9 @@ def measure(args, name, w, steps, warmup, preroll, world=1, rank=0, local=0, cpu
             * prof["cells_per_block"]
     else:
         alg = per_cell * prof["active_blocks"] * prof["cells_per_block"]
-    # average launch duration of the dominant kernel: when a step is that kernel (with its tile
-    # scan, about 3 % of the step, where it has one), the timed region itself (K steps between
-    # two events); otherwise its per-launch events
+    # average duration of the stencil kernels: when a step is them alone (with the scan in front of
+    # them, where there is one), the timed region itself (K steps between two events); otherwise
+    # their per-launch events
     if step_is_stencil(w):
         kernel_ms = ms / max(1, steps)
         alg_per_launch = cells * per_cell / max(1, steps) if w["model"] != "dendrite" else alg / nprof
@@ -322,6 +322,7 @@ def measure(args, name, w, steps, warmup, preroll, world=1, rank=0, local=0, cpu
     res = None
     if rank == 0:
         total_blocks = sim.info.nb
+        launches = step_launches(w, sim.info.grid_ctas)
         res = {
             "value": cells_all / (t_max * 1e-3), "unit": "cell-updates/s", "steps": steps, "warmup": warmup,
             "ms_per_step": t_max / steps, "dtype": "f32" if w["precision"] else "f64",
@@ -341,8 +342,7 @@ def measure(args, name, w, steps, warmup, preroll, world=1, rank=0, local=0, cpu
                          "frac": achieved / peak if peak else None, "traffic": traffic,
                          "kernel": f"{w['model']}_step", "peak_kind": peak_kind,
                          "alg_bytes_per_active_cell": per_cell, "kernel_ms_avg": kernel_ms,
-                         "kernel_timing": ("timed region, tile scan + tile kernel per step" if queue_path(w)
-                                           else "timed region, one launch per step") if step_is_stencil(w)
+                         "kernel_timing": "timed region, per step: " + " + ".join(launches) if step_is_stencil(w)
                          else "per-launch CUDA events",
                          "frac_of_8tbs_spec": achieved / 8000.0},
             "step_breakdown_ms": {"stencil": prof["stencil_ms"] / nprof, "reduce": prof["reduce_ms"] / nprof,
@@ -351,7 +351,7 @@ def measure(args, name, w, steps, warmup, preroll, world=1, rank=0, local=0, cpu
                          "dense_over_dba_time": dense_ms / dba_ms if dba_ms else None,
                          "dense_cell_updates_per_s": dense_cells / (dense_ms * 1e-3) if dense_ms else None,
                          "steps": ncmp, "timing": "captured graphs, CUDA events, same starting state"},
-            "gpu_launches": steps * launches_per_step(w),
+            "gpu_launches": steps * len(launches),
             "clocks": clk.summary(),
             "status": status,
         }
@@ -409,26 +409,22 @@ def run_ours(args, w):
     return result
 
 
-def kh_strips(w):
-    """KH workloads whose fully active tiles go by strips (FP32, 2^20 cells and more, not conserved)."""
-    return w["model"] == "kh" and w["precision"] == 1 and w["nx"] * w["ny"] >= 1 << 20 and not w["conserved"]
-
-
-def queue_path(w):
-    """Workloads whose step is a scan kernel listing the step's tiles and the tile kernel that
-    takes them (KH tiles, large FP32 3-D dendrite grids)."""
-    return w["model"] == "kh" or (w["model"] == "dendrite" and w["nz"] > 1 and w["precision"] == 1)
-
-
-def launches_per_step(w):
-    """This engine's kernel launches per step."""
-    if w["model"] == "kh":   # tile scan + (strips) + tile kernel (grids of 16-cell multiples, blocks 8 or 16)
-        return (3 if kh_strips(w) and w["mode"] else 2) + (2 if w["conserved"] else 0)
-    if queue_path(w):
-        return 2
-    if w["model"] == "modelb" and not (w["precision"] == 1 and w["nz"] == 1):
-        return 2 + (2 if w["conserved"] else 0)   # FP64 / 3-D: potentials, update (reduce, correct)
-    return 1       # FP32 2-D Model B: one kernel, the conserved reduction inside it
+def step_launches(w, grid_ctas):
+    """Names of this engine's kernel launches in a step (grid_ctas: dba_info's, for a 3-D dendrite
+    the CTAs on the GPU at once)."""
+    dba = bool(w["mode"])
+    correct = ["reduction", "correction"] if w["conserved"] and dba else []
+    if w["model"] == "kh":   # (grids of 16-cell multiples in blocks of 8 or 16)
+        strips = w["precision"] == 1 and w["nx"] * w["ny"] >= 1 << 20 and not (w["conserved"] and dba)
+        if strips:
+            return ["scan", "strips", "tiles"] if dba else ["scan", "strips"]
+        return ["scan", "tiles"] + correct
+    if w["model"] == "dendrite":   # 3-D: a list where a grid has more than four tiles per resident CTA
+        tiles = -(-w["nx"] // 32) * -(-w["ny"] // 8) * -(-w["nz"] // 8)
+        return ["scan", "tiles"] if w["nz"] > 1 and tiles > 4 * grid_ctas else ["step"]
+    if w["precision"] == 1 and w["nz"] == 1:
+        return ["step"]        # the conserved reduction inside it
+    return ["potentials", "update"] + correct
 
 
 def step_is_stencil(w):
