@@ -207,7 +207,6 @@ __global__ void __launch_bounds__(256, Den3<R, B>::MINB) dendrite3_step(GridP g,
     const int tid = threadIdx.x, nb = g.nb, w = tid >> 5;
     __shared__ uint4 s_mask;
     grid_wait();                                         // the scan, or the step before
-    if (LIST) grid_release();
     const int cnt = LIST ? (int)min(__ldcg(f.tctr), (unsigned)ntiles) : ntiles;
     if (LIST && blockIdx.x == 0 && tid == 0)             // the next step's count: the other of the pair
         *reinterpret_cast<unsigned*>(reinterpret_cast<uintptr_t>(f.tctr) ^ sizeof(unsigned)) = 0u;

@@ -247,7 +247,6 @@ __global__ void __launch_bounds__(256, 3) dendrite3_tile_step(GridP g, FlagP f, 
     // has ended at the one that opens tile i, where its bookkeeping runs (wake tests
     // double-buffered by tile parity), and the stage tile i + 1 refills is free there.
     grid_wait();                                 // the scan
-    grid_release();
     const int cnt = (int)min(__ldcg(f.tctr), (unsigned)(ntx * nty * (g.nz / B)));
     int k_pend = 0;
     auto entry = [&](int k, int slot) {

@@ -17,8 +17,9 @@ static int grid_of(const void* kern, size_t smem, int sms)
 // grid_wait here); captured into a graph as such.  A kernel that does not release lets the next
 // one in as its last CTAs end: us per step, plain / so: 512^2 FP64 dendrite 5.06 / 4.66, 256 x 200
 // FP64 Model B (two kernels) 7.7 / 7.05, 768^2 conserved (four) 48.8 / 47.9, 2048^2 FP32 39.1 / 39.0.
-// An early release only where the next kernel's CTAs are few or take tiles from a counter: others
-// crowd on the SMs that are free first (160^3 FP64 dendrite 13.8 / 15.0).
+// An early release only where the next kernel's CTAs take tiles from a counter and stay: others crowd on
+// the SMs that are free first (160^3 FP64 dendrite 13.8 / 15.0), and a small kernel let in early takes
+// their places (the scan beside the 512^3 FP32 dendrite's tiles 142.8 / 145.1).
 template <typename... K, typename... A>
 static cudaError_t launch_beside(void (*kernel)(K...), int grid, int threads, size_t smem, cudaStream_t st, A... args)
 {
