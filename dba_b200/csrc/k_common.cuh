@@ -165,9 +165,9 @@ __device__ __forceinline__ void wake_faces_diag(const GridP& g, uint8_t* w, int 
 }
 
 // Tile queue of one step.  A scan kernel appends the step's listed tiles as (tile, meta)
-// pairs to f.tlist, counting in f.tctr[0] (one atomic per warp); the tile kernel's CTAs
-// take entries in any order through the counter f.tctr[1], so a CTA whose tiles are
-// cheap takes more of them; the last CTA to finish (ticket f.tctr[2]) zeroes the three
+// pairs to f.tlist, counting in f.tctr[0] (one atomic per warp); CTA c of the tile kernel
+// takes entry c, then further ones through the counter f.tctr[1] (from entry G on), so a CTA
+// whose tiles are cheap takes more of them; the last CTA to finish (ticket f.tctr[2]) zeroes the three
 // counters for the next step.  Every tile's result is independent of which CTA
 // computes it and when.
 __device__ __forceinline__ void tile_list_append(const FlagP& f, bool take, int tile, unsigned meta, unsigned cap)

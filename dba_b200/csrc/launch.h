@@ -61,7 +61,7 @@ cudaError_t launch_dendrite3_tiles(bool dba_mode, int grid, cudaStream_t st, con
 // FP32 2-D uses the fast kernels (lazy conserved correction, reduction fused):
 // the 32x32-cell tile kernel when `tiles` (see modelb_tiles_ok), else one block
 // at a time.  `lz` may be null for FP64.
-// tiles: 0 the one-block kernel, 1 the tile kernel with 16-byte cp.async staging, 2 the
+// tiles: 0 modelb_fast_step, 1 the tile kernel with 16-byte cp.async staging, 2 the
 // tile kernel with bulk-copy (TMA engine) staging
 template <typename R>
 cudaError_t launch_modelb(int D, int B, bool dba_mode, int grid, cudaStream_t st, const GridP& g, const FlagP& f,

@@ -87,14 +87,15 @@ typedef struct dba_config {
     double ic_radius, ic_width;/* dendrite tanh seed */
     int ic_corner;             /* dendrite tanh seed at cell (0,0,0) instead of the centre */
     double noise_amp, noise_amp_z; /* Model B: x,y and z uniform-noise amplitudes (0.05, 0.001) */
-    int tiles;                 /* 1 (default): tile kernels where the shape allows -- FP32 2-D Model B on 32x32
-                                  cells (block 8, 16 or 32; nx, ny multiples of 32, or at least 64
-                                  and 2^16 cells), KH on 16x16 cells (nx, ny
-                                  multiples of 16, block 8 or 16), FP32 3-D dendrite on 32x8x8 cells (block 8);
-                                  2: as 1, with the FP32 2-D Model B tiles staged by
+    int tiles;                 /* 1 (default): FP32 2-D Model B on 32x32-cell tiles (block 8, 16 or 32; nx, ny
+                                  multiples of 32, or at least 64 and 2^16 cells), KH on 16x16-cell tiles
+                                  (nx, ny multiples of 16, block 8 or 16; FP32 from 2^20 cells on with strips
+                                  beside them), large FP32 3-D dendrites in blocks of 8 on double-buffered
+                                  32x8x8-cell tiles; 2: as 1, with the FP32 2-D Model B tiles staged by
                                   bulk copies of the TMA engine (one per block segment of a staged row)
-                                  instead of 16-byte cp.async pieces; 0: the one-block kernels and the
-                                  four-stage KH kernels */
+                                  instead of 16-byte cp.async pieces; 0: FP32 2-D Model B one block at a time,
+                                  KH in four stages, 3-D dendrites on the general tiles.  Other models,
+                                  precisions and sizes take the same kernels whatever it is */
     double cfl;                /* KH: > 0 picks each step's dt = cfl * min(dx, dy) / max(c + |v|) on the device
                                   (tile kernel only); 0 (default): the fixed dt */
 } dba_config;
