@@ -53,16 +53,32 @@ bool shape_supported(int model, int D, int B)
     return false;
 }
 
+// Whether the two-kernel Model B step of a 2-D grid in 4^2 or 8^2 blocks takes tiles of 16 rows: where there are more
+// tiles of 8 rows than the GPU holds three times over (148 x 4).  Half the CTAs, and 18 staged rows for 16 instead of
+// 10 for 8.  FP64 us per step, 8 / 16 rows, every block active (2 % active): 1024^2 (4096 tiles) 57.0 / 48.3 (16.3 / 11.8),
+// 768^2 (2304) 33.2 / 29.0 (10.4 / 9.5), 640^2 (1600) 24.3 / 23.0 (7.9 / 9.4).
+template <int D, int B>
+static bool mb_tall(int nx, int ny)
+{
+    return D == 2 && B <= 8 && ((nx + 31) / 32) * ((ny + 7) / 8) > 1776;
+}
+
 // the two-kernel Model B step: shared-memory limits on the current device, and the grid of
 // the correction pass
+template <typename R, int D, int B, bool TALL>
+static void mb_limits()
+{
+    using S = MBShape<R, D, B, TALL>;
+    cudaFuncSetAttribute(modelb_mu<R, D, B, true, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    cudaFuncSetAttribute(modelb_mu<R, D, B, false, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    cudaFuncSetAttribute(modelb_update<R, D, B, true, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_cons);
+    cudaFuncSetAttribute(modelb_update<R, D, B, false, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+}
 template <typename R, int D, int B>
 static int mb_prepare(int sms)
 {
-    using S = MBShape<R, D, B>;
-    cudaFuncSetAttribute(modelb_mu<R, D, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
-    cudaFuncSetAttribute(modelb_mu<R, D, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
-    cudaFuncSetAttribute(modelb_update<R, D, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_cons);
-    cudaFuncSetAttribute(modelb_update<R, D, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem_mu);
+    mb_limits<R, D, B, false>();
+    if constexpr (D == 2 && B <= 8) mb_limits<R, D, B, true>();
     return grid_of<R>((const void*)cons_correct<R>, 0, sms);
 }
 
@@ -146,15 +162,15 @@ bool modelb_uses_fast(int D, int B)
 }
 
 // one CTA per tile; potentials, then the update
-template <typename R, int D, int B>
+template <typename R, int D, int B, bool TALL>
 static cudaError_t mb_split(bool dba_mode, cudaStream_t st, const GridP& g, const FlagP& f, const MBP<R>& P)
 {
-    using S = MBShape<R, D, B>;
+    using S = MBShape<R, D, B, TALL>;
     const int nt = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY) * (D == 3 ? (g.nz + S::TZ - 1) / S::TZ : 1);
     const size_t sc = P.conserved ? S::smem_cons : S::smem_mu;
-    const cudaError_t e = launch_beside(dba_mode ? modelb_mu<R, D, B, true> : modelb_mu<R, D, B, false>, nt, S::NT, S::smem_mu, st, g, f, P);
+    const cudaError_t e = launch_beside(dba_mode ? modelb_mu<R, D, B, true, TALL> : modelb_mu<R, D, B, false, TALL>, nt, S::NT, S::smem_mu, st, g, f, P);
     if (e != cudaSuccess) return e;
-    return launch_beside(dba_mode ? modelb_update<R, D, B, true> : modelb_update<R, D, B, false>, nt, S::NT, dba_mode ? sc : S::smem_mu, st, g, f, P);
+    return launch_beside(dba_mode ? modelb_update<R, D, B, true, TALL> : modelb_update<R, D, B, false, TALL>, nt, S::NT, dba_mode ? sc : S::smem_mu, st, g, f, P);
 }
 
 template <typename R>
@@ -180,7 +196,9 @@ cudaError_t launch_modelb(int D, int B, bool dba_mode, int grid, cudaStream_t st
     }
 #define XM(d, b)                                                                            \
     if constexpr (!(sizeof(R) == 4 && d == 2))                                              \
-        if (D == d && B == b) return mb_split<R, d, b>(dba_mode, st, g, f, P);
+        if (D == d && B == b)                                                               \
+            return mb_tall<d, b>(g.nx, g.ny) ? mb_split<R, d, b, d == 2 && b <= 8>(dba_mode, st, g, f, P) \
+                                             : mb_split<R, d, b, false>(dba_mode, st, g, f, P);
     DBA_MB_SHAPES(XM)
 #undef XM
     (void)lz;

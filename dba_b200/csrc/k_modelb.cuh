@@ -37,11 +37,9 @@
 // 64 registers leave four CTAs per SM: 3 CTAs at 80 registers took 792 us where 4 take 708.
 // Measured per step, every block active, before -> now: 256^3 FP64 in 4^3 blocks 5167 ->
 // 708 us, 192^3 FP32 in 8^3 blocks (regular) 554 -> 168 us, 4^3 blocks 1088 -> 187 us;
-// 768^2 FP64 in 4^2 blocks 72.9 -> 33.5 us, conserved in 16^2 blocks 67.5 -> 47.9 us.  A 2-D grid of
+// 768^2 FP64 in 4^2 blocks 72.7 -> 29.0 us, conserved in 16^2 blocks 67.5 -> 47.9 us.  A 2-D grid of
 // many tiles that is nearly all asleep was faster one block at a time (idle CTAs of two
-// kernels): 1024^2 in 4^2 blocks 2 % active 10.0 -> 16.3, 12 % 20.5 -> 24.0, 43 % 62 -> 36.
-// Several tiles per CTA, their flags read at once, took 13.2 and 20.6 there, but 38.1 at 43 %
-// and two registers more than all other grids have.
+// kernels): 1024^2 in 4^2 blocks 2 % active 10.1 -> 11.8, 12 % 20.5 -> 19.0, 43 % 62 -> 33.
 // The Nz == 1 form keeps the reference's 27-term sum with the z neighbours
 // wrapped onto the cell itself.
 #pragma once
@@ -132,10 +130,11 @@ struct LapZ {
 // a tile holds whole blocks, and the staged box of three fields leaves room for 4 CTAs of
 // 256 threads (modelb_mu at 32 x 8 x 8 in FP64: 86 KB, 2 CTAs, and half the speed; FP32 8^3
 // with 4 cells per thread and CTAs of 512: 223 us where 8 cells and 256 threads take 168).
-template <typename R, int D, int B>
+// 2-D: 32 x 8 (4^2, 8^2 blocks), TALL 32 x 16 (mb_tall), 32 x 16 or 32 x 32 (16^2, 32^2 blocks).
+template <typename R, int D, int B, bool TALL = false>
 struct MBShape {
     static constexpr int TX = D == 3 && B == 8 && sizeof(R) == 8 ? 16 : 32;
-    static constexpr int TY = D == 3 ? 8 : (B > 8 ? B : 8), TZ = D == 3 ? B : 1;   // tile in cells
+    static constexpr int TY = D == 3 ? 8 : (B > 8 ? B : (TALL ? 16 : 8)), TZ = D == 3 ? B : 1;   // tile in cells
     static constexpr int NBX = TX / B, NBY = TY / B, NBZ = D == 3 ? TZ / B : 1, NBT = NBX * NBY * NBZ;
     static constexpr int RX = NBX + 2, RY = NBY + 2, RZ = D == 3 ? NBZ + 2 : 1, NR = RX * RY * RZ;
     static constexpr int PC = 16 / (int)sizeof(R);       // cells per staged piece (B is a multiple)
@@ -282,10 +281,10 @@ __device__ __forceinline__ void column_laps(const R* s, R inv_dx2, R* lap)
     }
 }
 
-template <typename R, int D, int B, bool DBA>
-__global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MINB)) modelb_mu(GridP g, FlagP f, MBP<R> P)
+template <typename R, int D, int B, bool DBA, bool TALL>
+__global__ void __launch_bounds__((MBShape<R, D, B, TALL>::NT), (MBShape<R, D, B, TALL>::MINB)) modelb_mu(GridP g, FlagP f, MBP<R> P)
 {
-    using S = MBShape<R, D, B>;
+    using S = MBShape<R, D, B, TALL>;
     constexpr int NC = S::NC, SW = S::SW, PL = S::PL, SV = S::SV, NT = S::NT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* stage = reinterpret_cast<R*>(smem_raw);           // [x, y, z][SD][SH][SW]
@@ -396,10 +395,10 @@ __global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MIN
     }
 }
 
-template <typename R, int D, int B, bool DBA>
-__global__ void __launch_bounds__((MBShape<R, D, B>::NT), (MBShape<R, D, B>::MINB)) modelb_update(GridP g, FlagP f, MBP<R> P)
+template <typename R, int D, int B, bool DBA, bool TALL>
+__global__ void __launch_bounds__((MBShape<R, D, B, TALL>::NT), (MBShape<R, D, B, TALL>::MINB)) modelb_update(GridP g, FlagP f, MBP<R> P)
 {
-    using S = MBShape<R, D, B>;
+    using S = MBShape<R, D, B, TALL>;
     constexpr int NC = S::NC, SW = S::SW, PL = S::PL, SV = S::SV;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* stage = reinterpret_cast<R*>(smem_raw);           // [x, y, z potentials][SD][SH][SW]
